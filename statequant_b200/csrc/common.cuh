@@ -19,6 +19,13 @@ constexpr float FP16_TINY = 5.960464477539063e-08f;   // 2^-24
 constexpr float FP16_MIN_NORMAL = 6.103515625e-05f;   // 2^-14
 constexpr float MAGIC = 12582912.0f;                  // 1.5 * 2^23: adding it rounds to an integer (half-even)
 
+// Programmatic dependent launch: every kernel of this library is launched so that its CTAs may become resident while the
+// kernel in front of it on the stream still runs (launch_pdl in launchers.h).  dependency_wait() stands in front of a
+// kernel's first access to global memory and returns once that kernel has finished and its writes are visible;
+// dependency_release(), after it, lets the next kernel's CTAs in as soon as all of this one's are resident.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 enum { DT_F32 = 0, DT_BF16 = 1, DT_F16 = 2 };
 enum { K_GDN = 0, K_M2 = 1, K_KDA = 2 };
 

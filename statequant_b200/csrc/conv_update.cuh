@@ -97,6 +97,8 @@ template <int DTX, int DTW, int W, int LAY>
 #define SQB_CONV_MINB 1
 #endif
 __global__ void __launch_bounds__(NT, SQB_CONV_MINB) conv_update_vec(const __grid_constant__ ConvArgs A) {
+  dependency_wait();
+  dependency_release();
   constexpr int ESZ = DTX == DT_F32 ? 4 : 2, WSZ = DTW == DT_F32 ? 4 : 2;
   constexpr int VEC = 16 / ESZ, T = W - 1, XW = 4;           // XW: 32-bit words of a 16-byte piece
   constexpr bool TYPED = ESZ == 2 && WSZ == 2;
@@ -191,6 +193,8 @@ __global__ void __launch_bounds__(NT, SQB_CONV_MINB) conv_update_vec(const __gri
 
 // any strides, any state_len >= width - 1; one channel per thread.  grid: x = row, y = chunk of NT channels.
 __global__ void __launch_bounds__(NT) conv_update_any(const __grid_constant__ ConvArgs A) {
+  dependency_wait();
+  dependency_release();
   const int row = blockIdx.x, c = blockIdx.y * NT + threadIdx.x;
   if (c >= A.dim) return;
   const int line = conv_line(A, row);
@@ -228,17 +232,15 @@ inline int launch_conv_update(const ConvArgs& a, cudaStream_t stream) {
   if (vecok) {
     const dim3 grid(a.rows, (a.dim / vec + NT - 1) / NT);
 #define SQB_CONV_CASE(X, S, WW, L) \
-    if (a.dt_x == X && a.dt_w == S && W == WW && lay == L) conv_update_vec<X, S, WW, L><<<grid, NT, 0, stream>>>(a);
+    if (a.dt_x == X && a.dt_w == S && W == WW && lay == L) e = launch_pdl(conv_update_vec<X, S, WW, L>, grid, NT, 0, stream, a);
 #define SQB_CONV_W(X, S) SQB_CONV_CASE(X, S, 2, 0) SQB_CONV_CASE(X, S, 2, 1) SQB_CONV_CASE(X, S, 3, 0) \
     SQB_CONV_CASE(X, S, 3, 1) SQB_CONV_CASE(X, S, 4, 0) SQB_CONV_CASE(X, S, 4, 1)
     SQB_CONV_W(DT_BF16, DT_BF16) SQB_CONV_W(DT_F16, DT_F16) SQB_CONV_W(DT_BF16, DT_F32) SQB_CONV_W(DT_F16, DT_F32)
     SQB_CONV_W(DT_F32, DT_F32) SQB_CONV_W(DT_F32, DT_BF16) SQB_CONV_W(DT_F32, DT_F16)
 #undef SQB_CONV_W
 #undef SQB_CONV_CASE
-    e = cudaGetLastError();
   } else {
-    conv_update_any<<<dim3(a.rows, (a.dim + NT - 1) / NT), NT, 0, stream>>>(a);
-    e = cudaGetLastError();
+    e = launch_pdl(conv_update_any, dim3(a.rows, (a.dim + NT - 1) / NT), NT, 0, stream, a);
   }
   return e == cudaSuccess ? 0 : -(1000 + static_cast<int>(e));
 }

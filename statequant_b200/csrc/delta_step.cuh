@@ -173,6 +173,8 @@ __device__ __forceinline__ bool round_fast(const float2 (&x)[NP], float s, float
 
 template <int KIND, int BITS, bool AXK>
 __global__ void __launch_bounds__(NT) delta_step_kernel(const __grid_constant__ StepArgs A) {
+  dependency_wait();
+  dependency_release();
   using F = Fmt<BITS>;
   constexpr int CPL = F::CPL;            // columns per lane chunk
   constexpr int NP = CPL / 2;            // float2 pairs per chunk

@@ -67,6 +67,8 @@ struct FoldArgs {
 
 template <bool VDEC, int BITS, bool AXK, int LPR>
 __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ FoldArgs A, const __grid_constant__ SmemF P) {
+  dependency_wait();
+  dependency_release();
   constexpr int DK = LPR * 16;
   constexpr bool TENS_OK = !VDEC && AXK && LPR == 8;       // instantiations that carry the tensor-pipe fold
   extern __shared__ __align__(128) uint8_t smraw[];

@@ -37,8 +37,7 @@ int launch_fold_one(const StepArgs& a, cudaStream_t stream, float* out) {
   if (per_sm < 1) per_sm = 1;
   long long grid = static_cast<long long>(nsm) * per_sm;
   if (grid > pairs) grid = pairs;
-  kern<<<static_cast<unsigned>(grid), NT, plan.total, stream>>>(f, plan);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pdl(kern, dim3(static_cast<unsigned>(grid)), NT, plan.total, stream, f, plan);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
 }
@@ -75,8 +74,7 @@ int launch_write_one(int kind, const StepArgs& a, const float* X, cudaStream_t s
   w.gc_width = kind == K_KDA ? a.DK : 1;
   const long long ctas = static_cast<long long>(a.rows) * a.HV;
   if (ctas > 2147483647LL) return 1;
-  slot_write_kernel<BITS, AXK, LPR><<<static_cast<unsigned>(ctas), NT, 0, stream>>>(w);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pdl(slot_write_kernel<BITS, AXK, LPR>, dim3(static_cast<unsigned>(ctas)), NT, 0, stream, w);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
 }

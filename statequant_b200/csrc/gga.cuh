@@ -361,6 +361,8 @@ __host__ __device__ inline GgaSmem gga_smem(int dk, int dv, int M, int group) {
 // arithmetic folds into immediates for the usual 128 x 128 head
 template <int DKT, int DVT>
 __global__ void __launch_bounds__(GNT) gga_step_kernel(const __grid_constant__ GgaArgs A) {
+  dependency_wait();
+  dependency_release();
   extern __shared__ __align__(16) float gsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int dk = DKT ? DKT : A.DK, dv = DVT ? DVT : A.DV, M = A.M, HV = A.HV;
@@ -528,6 +530,8 @@ __global__ void __launch_bounds__(GNT) gga_step_kernel(const __grid_constant__ G
 
 // window counters, after every head of the slot has read them
 __global__ void gga_advance_kernel(uint8_t* blob, long long stride, const int* idx, int rows, int M) {
+  dependency_wait();
+  dependency_release();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= rows) return;
   const long long seq = idx[b];
@@ -540,6 +544,8 @@ __global__ void gga_advance_kernel(uint8_t* blob, long long stride, const int* i
 
 // fit + pack canonical states X [P, HV, dk, dv] into slots; zero the counters
 __global__ void __launch_bounds__(GNT) gga_store_kernel(const __grid_constant__ GgaArgs A) {
+  dependency_wait();
+  dependency_release();
   extern __shared__ __align__(16) float gsm[];
   const int tid = threadIdx.x;
   const int dk = A.DK, dv = A.DV, HV = A.HV;
@@ -559,6 +565,8 @@ __global__ void __launch_bounds__(GNT) gga_store_kernel(const __grid_constant__ 
 
 // unpack slots into canonical fp32 Y [P, HV, dk, dv] (the stored state, without the window)
 __global__ void __launch_bounds__(GNT) gga_load_kernel(const __grid_constant__ GgaArgs A) {
+  dependency_wait();
+  dependency_release();
   extern __shared__ __align__(16) float gsm[];
   const int tid = threadIdx.x;
   const int dk = A.DK, dv = A.DV, HV = A.HV;
@@ -578,6 +586,8 @@ __global__ void __launch_bounds__(GNT) gga_load_kernel(const __grid_constant__ G
 
 // STEP's dual-axis fit as a fake-quant pass: Y = fit(X), X / Y [B, H, dk, dv]
 __global__ void __launch_bounds__(GNT) stepquant_fit_kernel(const __grid_constant__ GgaArgs A) {
+  dependency_wait();
+  dependency_release();
   extern __shared__ __align__(16) float gsm[];
   const int tid = threadIdx.x;
   const int dk = A.DK, dv = A.DV, HV = A.HV;

@@ -10,8 +10,7 @@ int launch_gga_reg(const GgaArgs& a, long long ctas, cudaStream_t stream) {
   cudaError_t e = limit.ensure(gga_step_reg_kernel, plan.total);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   if (ctas <= 0) return 0;
-  gga_step_reg_kernel<<<static_cast<unsigned>(ctas), RNT, plan.total, stream>>>(a);
-  e = cudaGetLastError();
+  e = launch_pdl(gga_step_reg_kernel, dim3(static_cast<unsigned>(ctas)), RNT, plan.total, stream, a);
   return e == cudaSuccess ? 0 : -1000 - static_cast<int>(e);
 }
 }  // namespace sqb

@@ -512,6 +512,8 @@ __device__ __forceinline__ bool gga_reg_head(GgaRegCtx& C, const GgaArgs& A, flo
 #define SQB_GGA_REG_MINB 2
 #endif
 __global__ void __launch_bounds__(RNT, SQB_GGA_REG_MINB) gga_step_reg_kernel(const __grid_constant__ GgaArgs A) {
+  dependency_wait();
+  dependency_release();
   extern __shared__ __align__(128) uint8_t rsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int HV = A.HV, M = A.M;

@@ -90,8 +90,7 @@ int launch_mma_one_io(const StepArgs& a, cudaStream_t stream) {
   while ((1 << b.m_log2) < a.M) b.m_log2++;
   if (a.HV / b.hpc > 65535) return 1;
   const dim3 grid(static_cast<unsigned>(a.rows), static_cast<unsigned>(a.HV / b.hpc));
-  kern<<<grid, NT, plan.total, stream>>>(b, plan, nst);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pdl(kern, grid, NT, plan.total, stream, b, plan, nst);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
 }

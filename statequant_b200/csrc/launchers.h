@@ -23,6 +23,22 @@ struct SmemLimit {
     return e;
   }
 };
+// Launch with programmatic stream serialisation: the grid's CTAs may be scheduled before the kernel in front of it has
+// finished; the kernel itself waits for that (dependency_wait in common.cuh) before it touches memory.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 struct GgaArgs;
 // the GGA step with the tile in registers (gga_reg.cuh): 0, 1 = shape not taken, -1000 - cudaError
 int launch_gga_reg(const GgaArgs& a, long long ctas, cudaStream_t stream);

@@ -21,6 +21,8 @@ struct WriteArgs {
 
 template <int BITS, bool AXK, int LPR>
 __global__ void __launch_bounds__(NT) slot_write_kernel(const __grid_constant__ WriteArgs A) {
+  dependency_wait();
+  dependency_release();
   constexpr int DK = LPR * 16;
   constexpr int RPP = 32 / LPR;
   constexpr int CB = 16 * BITS / 8;

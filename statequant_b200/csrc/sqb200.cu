@@ -121,8 +121,7 @@ int launch_one(const sqb::StepArgs& a, cudaStream_t stream) {
   }
   const long long ctas = static_cast<long long>(a.rows) * a.HV;
   if (ctas > 2147483647LL) return fail(SQB_EINVAL, "rows * hv = %lld exceeds the grid limit", ctas);
-  kern<<<static_cast<unsigned>(ctas), sqb::NT, smem, stream>>>(a);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = sqb::launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), sqb::NT, smem, stream, a);
   if (e != cudaSuccess) return fail(SQB_ECUDA, "kernel launch: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
@@ -424,8 +423,7 @@ int launch_gga(K kern, const sqb::GgaArgs& a, long long ctas, cudaStream_t strea
   cudaError_t e = limit.ensure(kern, smem);
   if (e != cudaSuccess) return fail(SQB_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   if (ctas <= 0) return 0;
-  kern<<<static_cast<unsigned>(ctas), sqb::GNT, smem, stream>>>(a);
-  e = cudaGetLastError();
+  e = sqb::launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), sqb::GNT, smem, stream, a);
   if (e != cudaSuccess) return fail(SQB_ECUDA, "kernel launch: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
@@ -475,8 +473,8 @@ int sqb_gga_step(const sqb_gga_layout_t* L, const sqb_gdn_inputs_t* in, void* st
     }
   }
   if (L->pw) {
-    sqb::gga_advance_kernel<<<(in->rows + 127) / 128, 128, 0, st>>>(a.blob, a.stride, a.idx, in->rows, L->m);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = sqb::launch_pdl(sqb::gga_advance_kernel, dim3((in->rows + 127) / 128), 128, 0, st, a.blob, a.stride, a.idx,
+                                         static_cast<int>(in->rows), static_cast<int>(L->m));
     if (e != cudaSuccess) return fail(SQB_ECUDA, "kernel launch: %s", cudaGetErrorString(e));
     g_launches.fetch_add(1, std::memory_order_relaxed);
   }

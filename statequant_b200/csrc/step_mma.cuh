@@ -135,6 +135,8 @@ template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV = false, bool 
 __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((BITS == 8 && UPG == 1) || (BITS == 4 && UPG == 2)) ? SQB_MMA_MINB_TFOLD : SQB_MMA_MINB_FOLD))
                                                : (BITS == 4 ? SQB_MMA_MINB4 : SQB_MMA_MINB8))
     step_mma_kernel(const __grid_constant__ StepArgs A, const __grid_constant__ SmemM P, const int nst) {
+  dependency_wait();
+  dependency_release();
   constexpr int DK = 128, NG = 4 / UPG, G = 32 * UPG;
   constexpr bool V8 = AXV && BITS == 8;          // 32 pieces of 4 rows instead of 8 pieces of 16
   constexpr int ROWB = DK * BITS / 8, PROWS = V8 ? V8_PIECE_ROWS : 16, PITCH = PROWS * ROWB + 16;

@@ -266,6 +266,8 @@ namespace sqb {
 template <int KIND, int BITS, bool AXK, int LPR>
 __global__ void __launch_bounds__(NT, AXK ? (KIND == K_M2 ? SQB_MINB_K_M2 : SQB_MINB_K) : SQB_MINB) step_tma_kernel(const __grid_constant__ StepArgs A, const __grid_constant__ Smem2 P,
                                                                 const int nst) {
+  dependency_wait();
+  dependency_release();
   constexpr int DK = LPR * 16;
   constexpr int RPP = 32 / LPR;                  // rows per warp pass
   constexpr int CW = DK / 32;                    // columns per lane in the prologue
