@@ -141,6 +141,185 @@ __device__ __forceinline__ void fold_left(const int8_t* ub, float uq, const floa
   A1 = bf2(p1[0], p1[1]); A2 = bf2(p2[0], p2[1]); A3 = bf2(p3[0], p3[1]);
 }
 
+// The values of NH halves (32 columns each) of two rows from half h0 on, advanced across the buffer, as accumulators
+// acc[half][N-block][row pair].  m: the two rows' codes as fragment registers (8-bit: (row a, row b) x two words; 4-bit: (row
+// a, row b)); sc: their scales by group; A1 .. A3: the A fragments of L (fold_left); al2 / ae: the decay (VDEC: per channel).
+template <int BITS, int UPG, int NH, bool VDEC>
+__device__ __forceinline__ void fold_acc(const uint32_t (&m)[NH][4], const float (&sc)[2][UPG == 1 ? NH : 1], const uint32_t (&A1)[2],
+                                         const uint32_t (&A2)[2], const uint32_t (&A3)[2], const uint32_t* KBf, int h0, int lane,
+                                         float2 al2, const float* ae, float (&acc)[NH][4][4]) {
+  [[maybe_unused]] const int t = lane & 3;
+  // ---- start values: (code * scale) * decay; code * scale is exact in fp32, so this rounds once, as the reference's
+  // two multiplications do ----
+#pragma unroll
+  for (int h = 0; h < NH; h++) {
+    const float s0 = sc[0][UPG == 1 ? h : 0], s1 = sc[1][UPG == 1 ? h : 0];
+    auto decay_of = [&](int p) -> float2 {         // of N-block p's column pair: per head, or (KDA) per key channel
+      if constexpr (VDEC) return *reinterpret_cast<const float2*>(ae + fold_col<BITS>(h0 + h, p, t));
+      else return al2;
+    };
+    if constexpr (BITS == 8) {
+      // byte u = code + 128 lands in bits 8..15 of 2^23's mantissa: the float is 2^23 + 256 u, and
+      // fma(that, scale / 256, -(2^23 + 2^15) scale / 256) is code * scale with every intermediate exact
+      const float q0 = s0 * 0.00390625f, q1 = s1 * 0.00390625f;
+      const float2 m0 = make_float2(q0, q0), m1 = make_float2(q1, q1);
+      const float2 c0 = make_float2(-8421376.0f * q0, -8421376.0f * q0), c1 = make_float2(-8421376.0f * q1, -8421376.0f * q1);
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const uint32_t wa = m[h][2 * (p >> 1)] ^ 0x80808080u, wb = m[h][2 * (p >> 1) + 1] ^ 0x80808080u;
+        float2 a, c;
+        if (p & 1) {
+          a = make_float2(__uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7424)), __uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7434)));
+          c = make_float2(__uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7424)), __uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7434)));
+        } else {
+          a = make_float2(__uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7404)), __uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7414)));
+          c = make_float2(__uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7404)), __uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7414)));
+        }
+        a = __fmul2_rn(__ffma2_rn(a, m0, c0), decay_of(p));
+        c = __fmul2_rn(__ffma2_rn(c, m1, c1), decay_of(p));
+        acc[h][p][0] = a.x; acc[h][p][1] = a.y; acc[h][p][2] = c.x; acc[h][p][3] = c.y;
+      }
+    } else {
+      // nibble n of a word is masked IN PLACE into 2^23's mantissa (n <= 4; nibbles 5, 6, 7 from the word shifted down
+      // by 20): the float is 2^23 + u 16^e, minus (2^23 + 8 16^e) gives (u - 8) 16^e exactly, and the power of
+      // sixteen goes into the scale.  Byte i of a word holds the pair (e, e') = (0,1), (2,3), (4,0), (1,2).
+      constexpr float E0[4] = {1.0f, 256.0f, 65536.0f, 16.0f}, E1[4] = {16.0f, 4096.0f, 1.0f, 256.0f};
+      const uint32_t w0 = m[h][0], w1 = m[h][1], w0s = w0 >> 20, w1s = w1 >> 20;
+      const uint32_t K = 0x4B000000u;
+      const float2 a[4] = {make_float2(nib_f<0x0000000Fu>(w0, K), nib_f<0x000000F0u>(w0, K)),
+                           make_float2(nib_f<0x00000F00u>(w0, K), nib_f<0x0000F000u>(w0, K)),
+                           make_float2(nib_f<0x000F0000u>(w0, K), nib_f<0x0000000Fu>(w0s, K)),
+                           make_float2(nib_f<0x000000F0u>(w0s, K), nib_f<0x00000F00u>(w0s, K))};
+      const float2 c[4] = {make_float2(nib_f<0x0000000Fu>(w1, K), nib_f<0x000000F0u>(w1, K)),
+                           make_float2(nib_f<0x00000F00u>(w1, K), nib_f<0x0000F000u>(w1, K)),
+                           make_float2(nib_f<0x000F0000u>(w1, K), nib_f<0x0000000Fu>(w1s, K)),
+                           make_float2(nib_f<0x000000F0u>(w1s, K), nib_f<0x00000F00u>(w1s, K))};
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const float2 bias = make_float2(-(8388608.0f + 8.0f * E0[p]), -(8388608.0f + 8.0f * E1[p]));
+        const float2 f0 = make_float2(s0 / E0[p], s0 / E1[p]), f1 = make_float2(s1 / E0[p], s1 / E1[p]);   // powers of two: exact
+        const float2 av = __fmul2_rn(__fmul2_rn(__fadd2_rn(a[p], bias), f0), decay_of(p));
+        const float2 cv = __fmul2_rn(__fmul2_rn(__fadd2_rn(c[p], bias), f1), decay_of(p));
+        acc[h][p][0] = av.x; acc[h][p][1] = av.y; acc[h][p][2] = cv.x; acc[h][p][3] = cv.y;
+      }
+    }
+  }
+  // ---- the eight buffer slots ----
+#pragma unroll
+  for (int h = 0; h < NH; h++) {
+    const uint32_t* kb = KBf + ((h0 + h) * 32 + lane) * 4;
+    const uint4 k1 = *reinterpret_cast<const uint4*>(kb);
+    const uint32_t r1[4] = {k1.x, k1.y, k1.z, k1.w};
+    if constexpr (VDEC) {
+      const uint4 k2 = *reinterpret_cast<const uint4*>(kb + 512), k3 = *reinterpret_cast<const uint4*>(kb + 1024);
+      const uint32_t r2[4] = {k2.x, k2.y, k2.z, k2.w}, r3[4] = {k3.x, k3.y, k3.z, k3.w};
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        mma_bf16(acc[h][p], A1[0], A1[1], A1[0], A1[1], r1[p], r2[p]);      // p1 r1 + p1 r2
+        mma_bf16(acc[h][p], A2[0], A2[1], A1[0], A1[1], r1[p], r3[p]);      // p2 r1 + p1 r3
+        mma_bf16(acc[h][p], A2[0], A2[1], A3[0], A3[1], r2[p], r1[p]);      // p2 r2 + p3 r1
+      }
+    } else {
+#pragma unroll
+      for (int p = 0; p < 4; p++) mma_bf16(acc[h][p], A1[0], A1[1], A2[0], A2[1], r1[p], r1[p]);
+#pragma unroll
+      for (int p = 0; p < 4; p++) mma_bf16_k8(acc[h][p], A3[0], A3[1], r1[p]);
+    }
+  }
+}
+// The fresh scales of the two rows' groups and the rounded codes, in the layout fold_acc took them.  Returns the scale that
+// lane t of the quad owns: row t & 1 of group t >> 1 (one group: lanes 2 and 3 hold copies).
+template <int BITS, int UPG, int NH>
+__device__ __forceinline__ float fold_round(const float (&acc)[NH][4][4], int lane, uint32_t (&o)[NH][4]) {
+  constexpr int NS = UPG == 1 ? NH : 1;
+  constexpr float QMAX = BITS == 4 ? 7.0f : 127.0f, MB = BITS == 4 ? MAGIC + 8.0f : MAGIC;
+  const int t = lane & 3;
+  // ---- fresh scales: absolute maxima over (row, group), index 2 group + row, over the quad ----
+  float mx[2 * NS];
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+      float v = 0.f;
+#pragma unroll
+      for (int h = 0; h < NH / NS; h++) {
+#pragma unroll
+        for (int p = 0; p < 4; p++) v = max3_abs(v, acc[s * (NH / NS) + h][p][2 * r], acc[s * (NH / NS) + h][p][2 * r + 1]);
+      }
+      mx[2 * s + r] = v;
+    }
+  }
+  float am;                                        // lane t of the quad: index t (two maxima: t & 1)
+  if constexpr (NS == 2) {
+    const bool up = (t & 2) != 0;
+    const float x0 = __shfl_xor_sync(0xffffffffu, up ? mx[0] : mx[2], 2), x1 = __shfl_xor_sync(0xffffffffu, up ? mx[1] : mx[3], 2);
+    mx[0] = fmaxf(up ? mx[2] : mx[0], x0);
+    mx[1] = fmaxf(up ? mx[3] : mx[1], x1);
+  }
+  am = fmaxf((t & 1) ? mx[1] : mx[0], __shfl_xor_sync(0xffffffffu, (t & 1) ? mx[0] : mx[1], 1));
+  if constexpr (NS == 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
+  const float s_own = fp16_scale(am, QMAX);
+  const bool fin = s_own <= 65504.0f;
+  const float r_own = fin ? __frcp_rn(s_own) : 0.f, n_own = fin ? -s_own : 0.f;
+  const bool tiny = __any_sync(0xffffffffu, s_own < FP16_MIN_NORMAL);
+  float rc[2][NS], ns[2][NS];
+#pragma unroll
+  for (int s = 0; s < NS; s++) {
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      rc[r][s] = __shfl_sync(0xffffffffu, r_own, (lane & 28) + 2 * s + r);
+      ns[r][s] = __shfl_sync(0xffffffffu, n_own, (lane & 28) + 2 * s + r);
+    }
+  }
+  // ---- round ----
+  float tv[NH][4][4];
+#pragma unroll
+  for (int h = 0; h < NH; h++) {
+    const int s = UPG == 1 ? h : 0;
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      const float2 a = div_round2(make_float2(acc[h][p][0], acc[h][p][1]), make_float2(rc[0][s], rc[0][s]), make_float2(ns[0][s], ns[0][s]), MB);
+      const float2 c = div_round2(make_float2(acc[h][p][2], acc[h][p][3]), make_float2(rc[1][s], rc[1][s]), make_float2(ns[1][s], ns[1][s]), MB);
+      tv[h][p][0] = a.x; tv[h][p][1] = a.y; tv[h][p][2] = c.x; tv[h][p][3] = c.y;
+    }
+  }
+  // only a scale in fp16's subnormal range (rounded far from absmax / qmax) lets a quotient round beyond qmax
+  if (tiny) {
+#pragma unroll
+    for (int h = 0; h < NH; h++) {
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) tv[h][p][e] = fminf(fmaxf(tv[h][p][e], MB - QMAX), MB + QMAX);
+      }
+    }
+  }
+  // ---- repack into the fragment registers ----
+  auto two = [](uint32_t a, uint32_t c) { return __byte_perm(a, c, 0x0040); };   // bytes (a, c)
+  auto u = [](float f) { return __float_as_uint(f); };
+#pragma unroll
+  for (int h = 0; h < NH; h++) {
+    const auto& v = tv[h];
+    if constexpr (BITS == 8) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int p = i & 2, e = (i & 1) * 2;
+        o[h][i] = __byte_perm(two(u(v[p][e]), u(v[p][e + 1])), two(u(v[p + 1][e]), u(v[p + 1][e + 1])), 0x5410);
+      }
+    } else {
+      // a candidate's low 4 bits are code + 8 and the next 4 are zero, so lo + 16 hi has the packed byte at the bottom
+      auto by = [](float lo, float hi) { return __float_as_uint(lo) + (__float_as_uint(hi) << 4); };
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int e = 2 * i;
+        o[h][i] = __byte_perm(two(by(v[0][e], v[0][e + 1]), by(v[1][e], v[1][e + 1])),
+                              two(by(v[2][e], v[2][e + 1]), by(v[3][e], v[3][e + 1])), 0x5410);
+      }
+    }
+  }
+  return s_own;
+}
+
 // Folds the 32 rows of warp w (row blocks 2w and 2w + 1) of a stage of eight pieces of R rows.
 //   st_addr / scs: the stage's codes (padded pieces) and scales [row][NG] in shared memory, both rewritten in place
 //   ubt: the stage's buffered values [heads][8][DV] int8 (slots 0..6); udq: this token's rounded values [heads][DV]
@@ -154,13 +333,13 @@ __device__ __forceinline__ void fold_left(const int8_t* ub, float uq, const floa
 // Bound by instruction issue (with its share of the step around it).  Two halves (64 columns, 32 values of a thread) are
 // taken at once: independent chains for the scheduler, and the 2 or 4 fresh scales of a quad (rows x groups) are
 // reduced by a transposing butterfly, computed by ONE lane each and exchanged.  Rounding is a branch-free exact division
-// (div_round2).  FOLD_MEASURED
+// (div_round2).  Token that folds, 256 rows of 32 heads, 8-bit: 123 us (141 us one span at a time with a verified reciprocal);
+// 4-bit, 4096 rows, a slot in eight folding: 767 us (941).
 template <int BITS, int UPG, int DV, bool VDEC = false, bool READ = false, int DK = 128, int R = 16>
 __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short* scs, const int8_t* ubt, const float* udq,
                                                const float* tab, const float* ksf, const uint32_t* KBf, int w, int lane,
                                                const float* ae = nullptr, float* out = nullptr) {
   constexpr int NHALF = DK / 32, NG = (NHALF + UPG - 1) / UPG, ROWB = DK * BITS / 8, PITCH = R * ROWB + 16, TABW = 20;
-  constexpr float QMAX = BITS == 4 ? 7.0f : 127.0f, MB = BITS == 4 ? MAGIC + 8.0f : MAGIC;
   static_assert(UPG == 1 || UPG == 2, "a scale group is one or two halves");
   const int g = lane >> 2, t = lane & 3;
   const uint32_t lrow = st_addr + (lane & 7) * PITCH + ((lane >> 3) & 1) * ROWB + (lane >> 4) * 16;
@@ -200,83 +379,7 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
 #pragma unroll
       for (int s = 0; s < NS; s++) { sc[0][s] = h2f(srow[g0 + s]); sc[1][s] = h2f(srow[NG + g0 + s]); }
       float acc[NH][4][4];
-      // ---- start values: (code * scale) * decay; code * scale is exact in fp32, so this rounds once, as the reference's
-      // two multiplications do ----
-#pragma unroll
-      for (int h = 0; h < NH; h++) {
-        const float s0 = sc[0][UPG == 1 ? h : 0], s1 = sc[1][UPG == 1 ? h : 0];
-        auto decay_of = [&](int p) -> float2 {         // of N-block p's column pair: per head, or (KDA) per key channel
-          if constexpr (VDEC) return *reinterpret_cast<const float2*>(ae + fold_col<BITS>(h0 + h, p, t));
-          else return al2;
-        };
-        if constexpr (BITS == 8) {
-          // byte u = code + 128 lands in bits 8..15 of 2^23's mantissa: the float is 2^23 + 256 u, and
-          // fma(that, scale / 256, -(2^23 + 2^15) scale / 256) is code * scale with every intermediate exact
-          const float q0 = s0 * 0.00390625f, q1 = s1 * 0.00390625f;
-          const float2 m0 = make_float2(q0, q0), m1 = make_float2(q1, q1);
-          const float2 c0 = make_float2(-8421376.0f * q0, -8421376.0f * q0), c1 = make_float2(-8421376.0f * q1, -8421376.0f * q1);
-#pragma unroll
-          for (int p = 0; p < 4; p++) {
-            const uint32_t wa = m[h][2 * (p >> 1)] ^ 0x80808080u, wb = m[h][2 * (p >> 1) + 1] ^ 0x80808080u;
-            float2 a, c;
-            if (p & 1) {
-              a = make_float2(__uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7424)), __uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7434)));
-              c = make_float2(__uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7424)), __uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7434)));
-            } else {
-              a = make_float2(__uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7404)), __uint_as_float(__byte_perm(wa, 0x4B000000u, 0x7414)));
-              c = make_float2(__uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7404)), __uint_as_float(__byte_perm(wb, 0x4B000000u, 0x7414)));
-            }
-            a = __fmul2_rn(__ffma2_rn(a, m0, c0), decay_of(p));
-            c = __fmul2_rn(__ffma2_rn(c, m1, c1), decay_of(p));
-            acc[h][p][0] = a.x; acc[h][p][1] = a.y; acc[h][p][2] = c.x; acc[h][p][3] = c.y;
-          }
-        } else {
-          // nibble n of a word is masked IN PLACE into 2^23's mantissa (n <= 4; nibbles 5, 6, 7 from the word shifted down
-          // by 20): the float is 2^23 + u 16^e, minus (2^23 + 8 16^e) gives (u - 8) 16^e exactly, and the power of
-          // sixteen goes into the scale.  Byte i of a word holds the pair (e, e') = (0,1), (2,3), (4,0), (1,2).
-          constexpr float E0[4] = {1.0f, 256.0f, 65536.0f, 16.0f}, E1[4] = {16.0f, 4096.0f, 1.0f, 256.0f};
-          const uint32_t w0 = m[h][0], w1 = m[h][1], w0s = w0 >> 20, w1s = w1 >> 20;
-          const uint32_t K = 0x4B000000u;
-          const float2 a[4] = {make_float2(nib_f<0x0000000Fu>(w0, K), nib_f<0x000000F0u>(w0, K)),
-                               make_float2(nib_f<0x00000F00u>(w0, K), nib_f<0x0000F000u>(w0, K)),
-                               make_float2(nib_f<0x000F0000u>(w0, K), nib_f<0x0000000Fu>(w0s, K)),
-                               make_float2(nib_f<0x000000F0u>(w0s, K), nib_f<0x00000F00u>(w0s, K))};
-          const float2 c[4] = {make_float2(nib_f<0x0000000Fu>(w1, K), nib_f<0x000000F0u>(w1, K)),
-                               make_float2(nib_f<0x00000F00u>(w1, K), nib_f<0x0000F000u>(w1, K)),
-                               make_float2(nib_f<0x000F0000u>(w1, K), nib_f<0x0000000Fu>(w1s, K)),
-                               make_float2(nib_f<0x000000F0u>(w1s, K), nib_f<0x00000F00u>(w1s, K))};
-#pragma unroll
-          for (int p = 0; p < 4; p++) {
-            const float2 bias = make_float2(-(8388608.0f + 8.0f * E0[p]), -(8388608.0f + 8.0f * E1[p]));
-            const float2 f0 = make_float2(s0 / E0[p], s0 / E1[p]), f1 = make_float2(s1 / E0[p], s1 / E1[p]);   // powers of two: exact
-            const float2 av = __fmul2_rn(__fmul2_rn(__fadd2_rn(a[p], bias), f0), decay_of(p));
-            const float2 cv = __fmul2_rn(__fmul2_rn(__fadd2_rn(c[p], bias), f1), decay_of(p));
-            acc[h][p][0] = av.x; acc[h][p][1] = av.y; acc[h][p][2] = cv.x; acc[h][p][3] = cv.y;
-          }
-        }
-      }
-      // ---- the eight buffer slots ----
-#pragma unroll
-      for (int h = 0; h < NH; h++) {
-        const uint32_t* kb = KBf + ((h0 + h) * 32 + lane) * 4;
-        const uint4 k1 = *reinterpret_cast<const uint4*>(kb);
-        const uint32_t r1[4] = {k1.x, k1.y, k1.z, k1.w};
-        if constexpr (VDEC) {
-          const uint4 k2 = *reinterpret_cast<const uint4*>(kb + 512), k3 = *reinterpret_cast<const uint4*>(kb + 1024);
-          const uint32_t r2[4] = {k2.x, k2.y, k2.z, k2.w}, r3[4] = {k3.x, k3.y, k3.z, k3.w};
-#pragma unroll
-          for (int p = 0; p < 4; p++) {
-            mma_bf16(acc[h][p], A1[0], A1[1], A1[0], A1[1], r1[p], r2[p]);      // p1 r1 + p1 r2
-            mma_bf16(acc[h][p], A2[0], A2[1], A1[0], A1[1], r1[p], r3[p]);      // p2 r1 + p1 r3
-            mma_bf16(acc[h][p], A2[0], A2[1], A3[0], A3[1], r2[p], r1[p]);      // p2 r2 + p3 r1
-          }
-        } else {
-#pragma unroll
-          for (int p = 0; p < 4; p++) mma_bf16(acc[h][p], A1[0], A1[1], A2[0], A2[1], r1[p], r1[p]);
-#pragma unroll
-          for (int p = 0; p < 4; p++) mma_bf16_k8(acc[h][p], A3[0], A3[1], r1[p]);
-        }
-      }
+      fold_acc<BITS, UPG, NH, VDEC>(m, sc, A1, A2, A3, KBf, h0, lane, al2, ae, acc);
       if constexpr (READ) {
         float* o0 = out + (long long)row0 * DK;
 #pragma unroll
@@ -291,91 +394,9 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
         }
         return;
       }
-      // ---- fresh scales: absolute maxima over (row, group), index 2 group + row, over the quad ----
-      float mx[2 * NS];
-#pragma unroll
-      for (int r = 0; r < 2; r++) {
-#pragma unroll
-        for (int s = 0; s < NS; s++) {
-          float v = 0.f;
-#pragma unroll
-          for (int h = 0; h < NH / NS; h++) {
-#pragma unroll
-            for (int p = 0; p < 4; p++) v = max3_abs(v, acc[s * (NH / NS) + h][p][2 * r], acc[s * (NH / NS) + h][p][2 * r + 1]);
-          }
-          mx[2 * s + r] = v;
-        }
-      }
-      float am;                                        // lane t of the quad: index t (two maxima: t & 1)
-      if constexpr (NS == 2) {
-        const bool up = (t & 2) != 0;
-        const float x0 = __shfl_xor_sync(0xffffffffu, up ? mx[0] : mx[2], 2), x1 = __shfl_xor_sync(0xffffffffu, up ? mx[1] : mx[3], 2);
-        mx[0] = fmaxf(up ? mx[2] : mx[0], x0);
-        mx[1] = fmaxf(up ? mx[3] : mx[1], x1);
-      }
-      am = fmaxf((t & 1) ? mx[1] : mx[0], __shfl_xor_sync(0xffffffffu, (t & 1) ? mx[0] : mx[1], 1));
-      if constexpr (NS == 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-      const float s_own = fp16_scale(am, QMAX);
-      const bool fin = s_own <= 65504.0f;
-      const float r_own = fin ? __frcp_rn(s_own) : 0.f, n_own = fin ? -s_own : 0.f;
-      const bool tiny = __any_sync(0xffffffffu, s_own < FP16_MIN_NORMAL);
-      float rc[2][NS], ns[2][NS];
-#pragma unroll
-      for (int s = 0; s < NS; s++) {
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-          rc[r][s] = __shfl_sync(0xffffffffu, r_own, (lane & 28) + 2 * s + r);
-          ns[r][s] = __shfl_sync(0xffffffffu, n_own, (lane & 28) + 2 * s + r);
-        }
-      }
-      if (NS == 2 || t < 2) srow[(t & 1) * NG + g0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);   // (the old scales are in registers by now)
-      // ---- round ----
-      float tv[NH][4][4];
-#pragma unroll
-      for (int h = 0; h < NH; h++) {
-        const int s = UPG == 1 ? h : 0;
-#pragma unroll
-        for (int p = 0; p < 4; p++) {
-          const float2 a = div_round2(make_float2(acc[h][p][0], acc[h][p][1]), make_float2(rc[0][s], rc[0][s]), make_float2(ns[0][s], ns[0][s]), MB);
-          const float2 c = div_round2(make_float2(acc[h][p][2], acc[h][p][3]), make_float2(rc[1][s], rc[1][s]), make_float2(ns[1][s], ns[1][s]), MB);
-          tv[h][p][0] = a.x; tv[h][p][1] = a.y; tv[h][p][2] = c.x; tv[h][p][3] = c.y;
-        }
-      }
-      // only a scale in fp16's subnormal range (rounded far from absmax / qmax) lets a quotient round beyond qmax
-      if (tiny) {
-#pragma unroll
-        for (int h = 0; h < NH; h++) {
-#pragma unroll
-          for (int p = 0; p < 4; p++) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) tv[h][p][e] = fminf(fmaxf(tv[h][p][e], MB - QMAX), MB + QMAX);
-          }
-        }
-      }
-      // ---- repack into the fragment registers ----
       uint32_t o[NH][4];
-      auto two = [](uint32_t a, uint32_t c) { return __byte_perm(a, c, 0x0040); };   // bytes (a, c)
-      auto u = [](float f) { return __float_as_uint(f); };
-#pragma unroll
-      for (int h = 0; h < NH; h++) {
-        const auto& v = tv[h];
-        if constexpr (BITS == 8) {
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int p = i & 2, e = (i & 1) * 2;
-            o[h][i] = __byte_perm(two(u(v[p][e]), u(v[p][e + 1])), two(u(v[p + 1][e]), u(v[p + 1][e + 1])), 0x5410);
-          }
-        } else {
-          // a candidate's low 4 bits are code + 8 and the next 4 are zero, so lo + 16 hi has the packed byte at the bottom
-          auto by = [](float lo, float hi) { return __float_as_uint(lo) + (__float_as_uint(hi) << 4); };
-#pragma unroll
-          for (int i = 0; i < 2; i++) {
-            const int e = 2 * i;
-            o[h][i] = __byte_perm(two(by(v[0][e], v[0][e + 1]), by(v[1][e], v[1][e + 1])),
-                                  two(by(v[2][e], v[2][e + 1]), by(v[3][e], v[3][e + 1])), 0x5410);
-          }
-        }
-      }
+      const float s_own = fold_round<BITS, UPG, NH>(acc, lane, o);
+      if (NS == 2 || t < 2) srow[(t & 1) * NG + g0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);   // (the old scales are in registers by now)
       if constexpr (BITS == 8) {
 #pragma unroll
         for (int h = 0; h < NH; h++) stsm_x4(addr + 32 * h, o[h]);

@@ -39,9 +39,25 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, 
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
+// Shapes the register-tile step takes: bf16 states of d_k 128 and d_v 64 or 128; Gated DeltaNet states of d_k 96 and d_v 64,
+// 128 or 192 with 8-bit codes in key groups of 32 or 4-bit codes in key groups of 64; decays per head, int8 buffer of 8,
+// q / k per key head, a CTA's rows of one key head.  The rest (fp32 states, KDA, other dims) is the generic kernel's.
+inline bool reg_shape_ok(const StepArgs& a, int bits, bool axk, int kind) {
+  if (kind == K_KDA || !a.qbuf || a.M != 8 || (!a.per_key_head && a.HV != a.HK)) return false;
+  if (bits == 16) {
+    if (a.DK != 128 || (a.DV != 64 && a.DV != 128)) return false;
+  } else {
+    if (kind != K_GDN || !axk || a.DK != 96 || (a.DV != 64 && a.DV != 128 && a.DV != 192)) return false;
+    if (!((bits == 8 && a.group == 32) || (bits == 4 && a.group == 64))) return false;
+  }
+  const int hps = a.DV == 64 ? 2 : 1;
+  return (a.HV / a.HK) % hps == 0 && a.HV / hps <= 65535;
+}
 struct GgaArgs;
 // the GGA step with the tile in registers (gga_reg.cuh): 0, 1 = shape not taken, -1000 - cudaError
 int launch_gga_reg(const GgaArgs& a, long long ctas, cudaStream_t stream);
+// the step with the state held in registers (step_reg.cuh), on shapes that reg_shape_ok takes
+int launch_reg(int kind, const StepArgs& a, int bits, cudaStream_t stream);
 int launch_staged_gdn(const StepArgs& a, int bits, bool axk, cudaStream_t stream);
 int launch_staged_m2(const StepArgs& a, int bits, bool axk, cudaStream_t stream);
 int launch_staged_kda(const StepArgs& a, int bits, bool axk, cudaStream_t stream);

@@ -203,6 +203,7 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
       return rf <= 0 ? rf : fail(SQB_ECUDA, "fold kernel refused a checked shape");
     }
   }
+  if (path != 1 && sqb::reg_shape_ok(a, bits, axk, KIND)) return sub_rc(sqb::launch_reg(KIND, a, bits, stream));
   if (path != 1 && tma_ok(a, bits, axk, kda) && fold_fits(a, bits, axk, kda)) {
     // the staged kernel only appends on a slot's m-th token; the fold launch that follows it rewrites the state of
     // the heads whose buffer is full (the generic kernel folds inside its own launch)

@@ -1,0 +1,514 @@
+// The fused decode step with the state held in REGISTERS: bf16 states of d_k 128, and 4- / 8-bit states of d_k 96 scaled along
+// k (groups of 64 / 32, the last one short); decays per head (Gated DeltaNet; bf16: Mamba2 too), int8 buffer of 8, q / k per
+// key head.
+//
+// One CTA per (batch row, ROWS state rows), a thread per row: one head of d_v 128 or 192, two heads of d_v 64 (of one key
+// head).  Warp w owns rows 32 w .. 32 w + 31 = two blocks of 16; lane (g, t) = (lane / 4, lane % 4) loads rows g and g + 8 of
+// a block, columns 32 j + 8 t .. + 7 of every unit j of 32 columns: one load each (16 bytes of bf16, 8 of int8, 4 of int4),
+// all requested before anything waits.  A loaded word is a register of a matrix instruction's A fragment as it stands (the
+// order of the columns along the contraction is free as long as B follows it) and, on the token that folds, part of a C
+// fragment as well: the state is read once, never passes through shared memory and goes back by stores of the registers it
+// came into.
+//
+// Read-out, bf16: q and k are cut into three bf16 pieces each (8 + 8 + 8 mantissa bits: exact), the columns of B; every
+// product is exact and a unit of 32 columns is summed from zero by the tensor core, the units in fp32.  Columns 0, 1, 2 are
+// the pieces of q, 4, 5, 6 those of k, so that the thread pair t = 0, 1 holds the parts of q and t = 2, 3 those of k.
+// Integer states: the byte digits of mma_pass.cuh, exact integer sums.
+// Fold: fold_mma.cuh's (three bf16 pieces of L against the int8 key codes), accumulators started at decay * state.
+//
+// HBM-bound by intent: a CTA's whole state is in flight at once.  Measured per layer and token, generic kernel -> this one
+// (the generic kernel's CTA goes through six block reductions before its state pass and holds 12 warps per SM): bf16, 96 rows
+// of 32 heads of 128 x 128, 120 -> 31.6 us (18 us at the copy rate); 4-bit, 64 rows of 30 heads of 96 x 192, a slot in eight
+// folding, 103 -> 26.6 us.
+#pragma once
+#include "launchers.h"
+#include "step_tma.cuh"
+#include "fold_mma.cuh"
+
+namespace sqb {
+
+// CTAs per SM: bf16 holds 64 words of state per thread (128 registers), integer states 12 to 32 (80 registers)
+constexpr int reg_min_ctas(int bits, int threads) { return (bits == 16 ? 512 : 768) / threads; }
+
+// N words of a lane's slice of a unit: 4 (bf16), 2 (int8) or 1 (int4)
+template <int N>
+__device__ __forceinline__ void ld_words(uint32_t* r, const uint8_t* p) {
+  if constexpr (N == 4) { const uint4 v = *reinterpret_cast<const uint4*>(p); r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w; }
+  else if constexpr (N == 2) { const uint2 v = *reinterpret_cast<const uint2*>(p); r[0] = v.x; r[1] = v.y; }
+  else r[0] = *reinterpret_cast<const uint32_t*>(p);
+}
+template <int N>
+__device__ __forceinline__ void st_words(uint8_t* p, const uint32_t* r) {
+  if constexpr (N == 4) *reinterpret_cast<uint4*>(p) = make_uint4(r[0], r[1], r[2], r[3]);
+  else if constexpr (N == 2) *reinterpret_cast<uint2*>(p) = make_uint2(r[0], r[1]);
+  else *reinterpret_cast<uint32_t*>(p) = r[0];
+}
+
+// The gates of value head h (one lane per head calls it): g, beta | dt, gcur, exp(gcur), exp(g), gcur + g, D into o[0 .. 6].
+// In two steps, so that the loads of a warp are in flight before their first use.
+struct GateRaw { uint32_t r[4]; float gcur; };
+template <int KIND>
+__device__ __forceinline__ GateRaw gates_load(const StepArgs& A, int b, int h, const float* GCseq) {
+  GateRaw w;
+  w.r[0] = w.r[1] = w.r[2] = w.r[3] = 0u;
+  if (KIND == K_GDN) {
+    if (A.gate) {
+      w.r[0] = ld1_raw(A.a + (long long)b * A.sa, A.dt_ab, h); w.r[1] = ld1_raw(A.dt_bias, A.dt_dtb, h);
+      w.r[2] = ld1_raw(A.A_log, A.dt_alog, h);                 w.r[3] = ld1_raw(A.b + (long long)b * A.sb, A.dt_ab, h);
+    } else {
+      w.r[0] = ld1_raw(A.g + (long long)b * A.sg, A.dt_g, h);  w.r[1] = ld1_raw(A.beta + (long long)b * A.sbeta, A.dt_g, h);
+    }
+  } else {
+    w.r[0] = ld1_raw(A.g + (long long)b * A.sg, A.dt_g, h);
+    if (A.dt_bias) w.r[1] = ld1_raw(A.dt_bias, A.dt_dtb, h);
+    w.r[2] = ld1_raw(A.A_log, A.dt_alog, h);
+    if (A.beta) w.r[3] = ld1_raw(A.beta, A.dt_beta, h);
+  }
+  w.gcur = GCseq[h];
+  return w;
+}
+template <int KIND>
+__device__ __forceinline__ void gates_finish(const StepArgs& A, const GateRaw& w, float* o) {
+  float g, bt, Dv = 0.f;
+  if (KIND == K_GDN) {
+    if (A.gate) {
+      const float x = cvt_raw(w.r[0], A.dt_ab) + cvt_raw(w.r[1], A.dt_dtb);
+      const float sp = x <= 20.0f ? logf(1.0f + expf(x)) : x;
+      g = -expf(cvt_raw(w.r[2], A.dt_alog)) * sp;
+      bt = __fdiv_rn(1.0f, 1.0f + expf(-cvt_raw(w.r[3], A.dt_ab)));
+    } else {
+      g = cvt_raw(w.r[0], A.dt_g);
+      bt = cvt_raw(w.r[1], A.dt_g);
+    }
+  } else {
+    float dtv = cvt_raw(w.r[0], A.dt_g);
+    if (A.dt_bias) dtv = dtv + cvt_raw(w.r[1], A.dt_dtb);
+    if (A.dt_softplus) dtv = dtv <= 20.0f ? logf(1.0f + expf(dtv)) : dtv;
+    if (A.dt_clamp) dtv = fminf(fmaxf(dtv, A.dt_min), A.dt_max);
+    g = __fmul_rn(cvt_raw(w.r[2], A.dt_alog), dtv);
+    bt = dtv;
+    if (A.beta) Dv = cvt_raw(w.r[3], A.dt_beta);
+  }
+  o[0] = g; o[1] = bt; o[2] = w.gcur; o[3] = expf(w.gcur); o[4] = expf(g); o[5] = w.gcur + g; o[6] = Dv;
+}
+
+// the sum of a hi + mid + lo triple whose lower parts may be 0 * inf: a hi part that is not finite stands alone
+__device__ __forceinline__ float add_parts(float hi, float lo) { return fabsf(hi) <= 3.402823466e38f ? hi + lo : hi; }
+
+template <int KIND, int BITS, int DK, int DV, int HPS, bool BIO>
+__global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_reg_kernel(const __grid_constant__ StepArgs A) {
+  dependency_wait();
+  dependency_release();
+  constexpr int NT = HPS * DV, M = 8, WPH = DV / 32, NU = DK / 32, CW = 4, ROWB = DK * BITS / 8;
+  constexpr int WPU = BITS / 4, UPG = BITS == 4 ? 2 : 1, NG = BITS == 16 ? 1 : (NU + UPG - 1) / UPG;
+  constexpr bool TWO = KIND != K_M2, QUANT = BITS != 16;
+  __shared__ __align__(16) uint2 Bf[QUANT ? 1 : 2 * NU * 32];          // bf16: B fragments of the state pass (bf16 pieces)
+  __shared__ __align__(16) uint32_t Bf8[2 * 4 * 32];       // B fragments of byte codes (byte digits): key tile, int8 state
+  __shared__ __align__(16) uint32_t Bf4[BITS == 4 ? 2 * 4 * 32 : 1];   // B fragments of nibble codes
+  __shared__ __align__(16) uint32_t KBf[DK * 4];           // key fragments of the fold
+  __shared__ __align__(16) uint32_t Lp[NT * 12];          // the fold's L: per row three pieces of eight bf16
+  __shared__ __align__(16) int8_t kbt[M * DK];
+  __shared__ __align__(16) int8_t kcur[DK];
+  __shared__ __align__(16) float hd[HPS * HD_W];
+  __shared__ float2 dcu[HPS * M], dqk[M];
+  __shared__ float gbs[HPS * M], ksf[M], tab[HPS * 20], red[NT / 32], misc[8];
+
+  const int dt_qk = BIO ? static_cast<int>(DT_BF16) : A.dt_qk, dt_v = BIO ? static_cast<int>(DT_BF16) : A.dt_v,
+            dt_out = BIO ? static_cast<int>(DT_BF16) : A.dt_out;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int b = blockIdx.x, h0 = blockIdx.y * HPS, hk = h0 / A.gqa_full;
+  const bool first = h0 == hk * A.gqa_full;                // the CTA that appends the key head's key
+  const int osz = dt_size(dt_out);
+  // q and k leave before the slot index is known
+  Raw4 rq, rk;
+  rq.v = make_uint4(0u, 0u, 0u, 0u); rk.v = rq.v; rq.vec = false; rk.vec = false;
+  const bool has_col = lane * CW < DK;                     // warps 0 and 3: four columns per lane
+  if ((warp == 0 || warp == 3) && has_col) {
+    rq = ld4_raw(A.q + (long long)b * A.sq, dt_qk, (long long)hk * DK + lane * CW);
+    rk = ld4_raw(A.k + (long long)b * A.sk, dt_qk, (long long)hk * DK + lane * CW);
+  }
+  long long seq = b;
+  if (A.idx != nullptr) {
+    seq = A.idx[b];
+    if (seq <= 0) {
+      uint8_t* orow = A.out + (long long)b * A.so + (long long)h0 * DV * osz;
+      for (int v = tid; v < HPS * DV; v += NT) stf(orow, dt_out, v, 0.0f);
+      return;
+    }
+  }
+  int* NPseq = reinterpret_cast<int*>(A.NPTR + seq * A.sN);
+  uint8_t* KBh = A.KB + seq * A.sKB + (long long)hk * M * DK;
+  uint8_t* UBseq = A.UB + seq * A.sUB;
+  unsigned short* KBSh = reinterpret_cast<unsigned short*>(A.KBS + seq * A.sKBS) + hk * M;
+  unsigned short* UBSseq = reinterpret_cast<unsigned short*>(A.UBS + seq * A.sUBS);
+  float* GBseq = reinterpret_cast<float*>(A.GB + seq * A.sGB);
+  float* GCseq = reinterpret_cast<float*>(A.GCUR + seq * A.sGC);
+
+  // ---- every fetch: a role's small ones first (they head the serial chains), then the state, then the buffered values --
+  uint2 kw[NU];                                            // warp 0: slot g of the key tile, its 8 columns of every unit
+  float ksl = 0.f;
+  GateRaw gr;
+  int nraw = 0;
+  float gb0 = 0.f, gc0 = 0.f;
+  unsigned short us0 = 0;
+  if (warp == 0) {
+#pragma unroll
+    for (int u = 0; u < NU; u++) kw[u] = *reinterpret_cast<const uint2*>(KBh + g * DK + 32 * u + 8 * t);
+    ksl = h2f(KBSh[g]);
+  } else if (warp == 1) {
+    gr.r[0] = gr.r[1] = gr.r[2] = gr.r[3] = 0u; gr.gcur = 0.f;
+    if (lane < HPS) gr = gates_load<KIND>(A, b, h0 + lane, GCseq);
+  } else if (warp == 2) {
+    nraw = NPseq[h0];                                      // the heads of a slot advance together
+    if (lane < HPS * M) {
+      gb0 = GBseq[(long long)h0 * M + lane]; gc0 = GCseq[h0 + lane / M];
+      us0 = UBSseq[h0 * M + lane];
+    }
+  }
+  const int hw = warp / WPH, h = h0 + hw, rv0 = (warp % WPH) * 32;       // this warp's head and its first row in it
+  const long long row0 = (long long)h * DV + rv0 + g;      // row g of the warp's first block
+  uint8_t* Srow = A.S + seq * A.sS + row0 * ROWB + BITS * t;
+  uint32_t sw[2][2][NU * WPU];                             // [block][row g, row g + 8][unit, word]
+  unsigned short scr[2][2][NG];
+  unsigned short* SCrow = nullptr;
+  if (QUANT) SCrow = reinterpret_cast<unsigned short*>(A.SC + seq * A.sSC) + row0 * NG;
+#pragma unroll
+  for (int x = 0; x < 2; x++) {
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+#pragma unroll
+      for (int u = 0; u < NU; u++) ld_words<WPU>(&sw[x][r][u * WPU], Srow + (16 * x + 8 * r) * ROWB + 4 * BITS * u);
+      if constexpr (QUANT) {
+#pragma unroll
+        for (int i = 0; i < NG; i++) scr[x][r][i] = SCrow[(16 * x + 8 * r) * NG + i];
+      }
+    }
+  }
+  const int rv = rv0 + 8 * t + g;                          // the row this lane finishes: block t / 2, half t % 2
+  const uint32_t rvt = ld1_raw(A.v + (long long)b * A.sv, dt_v, (long long)h * DV + rv);
+  int8_t ub[M - 1];
+#pragma unroll
+  for (int i = 0; i < M - 1; i++) ub[i] = static_cast<int8_t>(UBseq[((long long)h * M + i) * DV + rv]);
+
+  // ---- prologue, by role ----------------------------------------------------------------------------------------
+  uint32_t kword = 0;                                      // warp 3: the key as it goes into the buffer
+  float kscale = 0.f;
+  if (warp == 0) {
+    float qr[CW], kr[CW];
+    cvt4_raw(rq, dt_qk, qr);
+    cvt4_raw(rk, dt_qk, kr);
+    if (KIND != K_M2) {
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < CW; j++) { s0 += qr[j] * qr[j]; s1 += kr[j] * kr[j]; }
+      s0 = warp_sum(s0);
+      s1 = warp_sum(s1);
+      const float nq = __fsqrt_rn(s0 + 1e-6f), nk = __fsqrt_rn(s1 + 1e-6f);
+#pragma unroll
+      for (int j = 0; j < CW; j++) { qr[j] = __fdiv_rn(qr[j], nq) * A.scale; kr[j] = __fdiv_rn(kr[j], nk); }
+    }
+    // bf16: the state pass's fragments: lane l's columns 4 l .. 4 l + 3 are step l / 8 * 2 + l % 2, thread (l % 8) / 2
+    if constexpr (!QUANT) {
+      uint2* bw = Bf + (2 * (lane >> 3) + (lane & 1)) * 32 + ((lane & 7) >> 1);
+#pragma unroll
+      for (int vec = 0; vec < 2; vec++) {
+        float p[3][CW];
+#pragma unroll
+        for (int j = 0; j < CW; j++) split3(vec ? kr[j] : qr[j], p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+          bw[(4 * vec + s) * 4] = s == 3 || (vec && !TWO) ? make_uint2(0u, 0u) : make_uint2(bf2(p[s < 3 ? s : 0][0], p[s < 3 ? s : 0][1]),
+                                                                                       bf2(p[s < 3 ? s : 0][2], p[s < 3 ? s : 0][3]));
+      }
+    }
+    // the buffered keys against q and k: integer digits (mma_pass.cuh), the key codes straight from the loads
+    float d = 0.f, mq = 0.f, mk = 0.f;
+#pragma unroll
+    for (int j = 0; j < CW; j++) {
+      d += kr[j] * qr[j];
+      mq = fmaxf(mq, fabsf(qr[j]));
+      mk = fmaxf(mk, fabsf(kr[j]));
+    }
+    mq = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mq)));
+    if (TWO) mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
+    const FxScale fq = fx30_scale(mq), fk = fx30_scale(mk);
+#pragma unroll
+    for (int vec = 0; vec < 2; vec++) {
+      uint32_t y[CW];
+#pragma unroll
+      for (int j = 0; j < CW; j++) y[j] = vec == 0 ? fx30_digits(qr[j], fq) : (TWO ? fx30_digits(kr[j], fk) : 0u);
+      const uint32_t t0 = __byte_perm(y[0], y[1], 0x5140), t1 = __byte_perm(y[2], y[3], 0x5140);
+      const uint32_t t2 = __byte_perm(y[0], y[1], 0x7362), t3 = __byte_perm(y[2], y[3], 0x7362);
+      const uint32_t W[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410),
+                             __byte_perm(t2, t3, 0x7632)};                 // W[s]: digit s of the four columns
+#pragma unroll
+      for (int s = 0; s < 4; s++) Bf8[(2 * (lane >> 3) + (lane & 1)) * 32 + (vec * 4 + 3 - s) * 4 + ((lane & 7) >> 1)] = W[s];
+      if constexpr (BITS == 4) put_b_words<4>(Bf4, lane, vec, y[0], y[1], y[2], y[3]);
+    }
+    d = warp_sum(d);
+    if (lane == 0) { misc[0] = d; misc[4] = fq.i1; misc[5] = fq.i2; misc[6] = fk.i1; misc[7] = fk.i2; }
+#pragma unroll
+    for (int u = 0; u < NU; u++) *reinterpret_cast<uint2*>(kbt + g * DK + 32 * u + 8 * t) = kw[u];
+    __syncwarp();
+    int acc[4] = {MAGIC_I, MAGIC_I, 0, 0};                 // fragment rows 8 .. 15 are empty
+#pragma unroll
+    for (int u = 0; u < NU; u++)
+      mma_i8<false>(acc, kw[u].x, 0u, kw[u].y, 0u, Bf8[(2 * u) * 32 + lane], Bf8[(2 * u + 1) * 32 + lane]);
+    const float wa = (t & 1) ? 256.0f : 16777216.0f, wb = (t & 1) ? 1.0f : 65536.0f;
+    float T = fmaf((__int_as_float(acc[0]) - 12582912.0f) * ksl, wa, ((__int_as_float(acc[1]) - 12582912.0f) * ksl) * wb);
+    T += __shfl_xor_sync(0xffffffffu, T, 1);
+    T = t < 2 ? (T * fq.i1) * fq.i2 : (T * fk.i1) * fk.i2;
+    if (t == 0) { dqk[g].x = T; ksf[g] = ksl; }
+    if (t == 2) dqk[g].y = T;
+  } else if (warp == 1) {
+    if (lane < HPS) gates_finish<KIND>(A, gr, hd + lane * HD_W);
+  } else if (warp == 2) {
+    const int n0 = nraw & (M - 1);
+    if (lane == 0) misc[1] = __int_as_float(n0);
+    if (lane < HPS * M) {
+      // dead entries may hold anything: they are selected away
+      dcu[lane] = (lane & (M - 1)) < n0 ? make_float2(expf(gc0 - gb0), h2f(us0)) : make_float2(0.f, 0.f);
+      gbs[lane] = gb0;
+    }
+  } else if (warp == 3) {
+    // the key, rounded: its normalisation is redone here (the arithmetic of warp 0, so the same bits)
+    float kr[CW];
+    cvt4_raw(rk, dt_qk, kr);
+    if (KIND != K_M2) {
+      float s1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < CW; j++) s1 += kr[j] * kr[j];
+      s1 = warp_sum(s1);
+      const float nk = __fsqrt_rn(s1 + 1e-6f);
+#pragma unroll
+      for (int j = 0; j < CW; j++) kr[j] = __fdiv_rn(kr[j], nk);
+    }
+    float mx = 0.f;
+#pragma unroll
+    for (int j = 0; j < CW; j++) mx = fmaxf(mx, fabsf(kr[j]));
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+    kscale = fp16_scale(mx, 127.0f);
+#pragma unroll
+    for (int j = 0; j < CW; j++) kword |= (static_cast<uint32_t>(static_cast<int>(rq_exact(kr[j], kscale, 127.0f))) & 0xFFu) << (8 * j);
+    if (has_col) *reinterpret_cast<uint32_t*>(kcur + lane * 4) = kword;
+    if (lane == 0) misc[2] = kscale;
+  }
+  __syncthreads();
+  const float kq = misc[0];
+  const int n0 = __float_as_int(misc[1]);                  // live buffer entries of this slot
+  const bool full = n0 == M - 1;                           // this token fills the buffer: fold after the read-out
+  if (warp == 3 && first) {
+    if (has_col) *reinterpret_cast<uint32_t*>(KBh + (long long)n0 * DK + lane * 4) = kword;
+    if (lane == 0) KBSh[n0] = f2h(kscale);
+  }
+
+  // ---- read-out ---------------------------------------------------------------------------------------------------
+  float y[2];                                              // block x: this thread pair's vector, half t % 2
+  if constexpr (!QUANT) {
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+      float2 s01 = make_float2(0.f, 0.f), s23 = s01;
+#pragma unroll
+      for (int u = 0; u < NU; u++) {
+        const uint2 b0 = Bf[(2 * u) * 32 + lane], b1 = Bf[(2 * u + 1) * 32 + lane];
+        const uint32_t *wa = &sw[x][0][u * WPU], *wc = &sw[x][1][u * WPU];
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16(acc, wa[0], wc[0], wa[1], wc[1], b0.x, b0.y);
+        mma_bf16(acc, wa[2], wc[2], wa[3], wc[3], b1.x, b1.y);
+        s01 = __fadd2_rn(s01, make_float2(acc[0], acc[1]));
+        s23 = __fadd2_rn(s23, make_float2(acc[2], acc[3]));
+      }
+      // t even: (hi, mid); t odd: (lo, -).  The even lane of a pair ends up with row g, the odd one with row g + 8.
+      const float v0 = (t & 1) ? s01.x : add_parts(s01.x, s01.y), v1 = (t & 1) ? s23.x : add_parts(s23.x, s23.y);
+      const float own = (t & 1) ? v1 : v0, recv = __shfl_xor_sync(0xffffffffu, (t & 1) ? v0 : v1, 1);
+      y[x] = (t & 1) ? add_parts(recv, own) : add_parts(own, recv);
+    }
+  } else {
+    uint32_t bf[2 * NU];
+#pragma unroll
+    for (int r = 0; r < 2 * NU; r++) bf[r] = (BITS == 4 ? Bf4 : Bf8)[r * 32 + lane];
+    int ci[NG][2];                                         // start values: nibbles carry an offset of 8 (mma_pass.cuh)
+#pragma unroll
+    for (int i = 0; i < NG; i++) {
+      int d[4] = {0, 0, 0, 0};
+      if constexpr (BITS == 4) {
+#pragma unroll
+        for (int u = i * UPG; u < (i + 1) * UPG && u < NU; u++)
+          mma_i8<true>(d, 0x01010101u, 0x01010101u, 0x01010101u, 0x01010101u, bf[2 * u], bf[2 * u + 1]);
+      }
+      ci[i][0] = MAGIC_I - 8 * d[0];
+      ci[i][1] = MAGIC_I - 8 * d[1];
+    }
+    const float i1 = t < 2 ? misc[4] : misc[6], i2 = t < 2 ? misc[5] : misc[7];
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+      float2 p01 = make_float2(0.f, 0.f), p23 = p01;
+#pragma unroll
+      for (int i = 0; i < NG; i++) {
+        int acc[4] = {ci[i][0], ci[i][1], ci[i][0], ci[i][1]};
+#pragma unroll
+        for (int u = i * UPG; u < (i + 1) * UPG && u < NU; u++) {
+          const uint32_t *wa = &sw[x][0][u * WPU], *wc = &sw[x][1][u * WPU];
+          if constexpr (BITS == 8)
+            mma_i8<false>(acc, wa[0], wc[0], wa[1], wc[1], bf[2 * u], bf[2 * u + 1]);
+          else
+            mma_i8<true>(acc, wa[0] & 0x0F0F0F0Fu, wc[0] & 0x0F0F0F0Fu, (wa[0] >> 4) & 0x0F0F0F0Fu, (wc[0] >> 4) & 0x0F0F0F0Fu,
+                         bf[2 * u], bf[2 * u + 1]);
+        }
+        const float sa = h2f(scr[x][0][i]), sc = h2f(scr[x][1][i]);
+        const float2 nm = make_float2(-12582912.0f, -12582912.0f);
+        p01 = __ffma2_rn(__fadd2_rn(make_float2(__int_as_float(acc[0]), __int_as_float(acc[1])), nm), make_float2(sa, sa), p01);
+        p23 = __ffma2_rn(__fadd2_rn(make_float2(__int_as_float(acc[2]), __int_as_float(acc[3])), nm), make_float2(sc, sc), p23);
+      }
+      const float p[4] = {p01.x, p01.y, p23.x, p23.y};
+      y[x] = (join_digits(p, t) * i1) * i2;                // powers of two: exact
+    }
+  }
+  float tq, tk;
+  {
+    const float recv = __shfl_xor_sync(0xffffffffu, t < 2 ? y[1] : y[0], 2);
+    tq = t < 2 ? y[0] : recv;
+    tk = t < 2 ? recv : y[1];
+  }
+  const float4 hda = *reinterpret_cast<const float4*>(hd + hw * HD_W), hdb = *reinterpret_cast<const float4*>(hd + hw * HD_W + 4);
+  const float vt = cvt_raw(rvt, dt_v);
+  tq = hda.w * tq;
+  tk = hda.w * tk;
+#pragma unroll
+  for (int i = 0; i < M - 1; i++) {
+    if (i < n0) {                                          // uniform; dead entries may hold garbage
+      const float2 du = dcu[hw * M + i], dd = dqk[i];
+      const float xb = static_cast<float>(ub[i]) * du.y;
+      tq = fmaf(xb, du.x * dd.x, tq);
+      if (TWO) tk = fmaf(xb, du.x * dd.y, tk);
+    }
+  }
+  float u, o;
+  if (KIND == K_GDN) {
+    u = hda.y * fmaf(-hdb.x, tk, vt);
+    o = fmaf(kq, u, hdb.x * tq);
+  } else {
+    u = hda.y * vt;                                        // dt
+    o = fmaf(kq, u, hdb.x * tq);
+    if (A.beta) o = fmaf(hdb.z, vt, o);
+  }
+  stf(A.out + (long long)b * A.so + (long long)h * DV * osz, dt_out, rv, o);
+  // largest |u| of the head (non-negative floats order like their bit patterns; a NaN ends up as the maximum)
+  const float um = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(u))));
+  if (lane == 0) red[warp] = um;
+  __syncthreads();
+
+  // ---- append at slot n0 ---------------------------------------------------------------------------------------------
+  float umax = red[hw * WPH];
+#pragma unroll
+  for (int w = 1; w < WPH; w++) umax = fmaxf(umax, red[hw * WPH + w]);
+  const float usc = fp16_scale(umax, 127.0f);
+  float cc = fmaf(u, rcp_approx(usc), MAGIC) - MAGIC;
+  const float rem = fmaf(-cc, usc, u);
+  if (!(fabsf(rem) < usc * 0.49998474f) || usc < FP16_MIN_NORMAL) cc = rq_exact(u, usc, 127.0f);
+  UBseq[((long long)h * M + n0) * DV + rv] = static_cast<uint8_t>(static_cast<int>(cc));
+  if (rv == 0) {
+    UBSseq[h * M + n0] = f2h(usc);
+    GBseq[(long long)h * M + n0] = hdb.y;
+    GCseq[h] = full ? 0.f : hdb.y;
+    NPseq[h] = full ? 0 : n0 + 1;
+  }
+  if (!full) return;
+
+  // ---- fold ------------------------------------------------------------------------------------------------------
+  if (tid < HPS * M) {                                     // per head: decays and value scales of the slots
+    const int i = tid & (M - 1), hq = tid / M;
+    const float gnew = hd[hq * HD_W + 5];
+    tab[hq * 20 + i] = i == M - 1 ? 1.0f : expf(gnew - gbs[tid]);
+    tab[hq * 20 + 8 + i] = dcu[tid].y;
+    if (i == 0) tab[hq * 20 + 16] = expf(gnew);
+  }
+  build_key_frags<4, DK>(KBf, kbt, kcur, tid);             // (columns in the order of the state's words)
+  __syncthreads();
+  {
+    // this lane's row of L, in pieces: slot pairs as bf16 words
+    const float* tb = tab + hw * 20;
+    uint32_t* lw = Lp + (warp * 32 + 8 * t + g) * 12;
+#pragma unroll
+    for (int s = 0; s < M; s += 2) {
+      const float L0 = tb[s] * (static_cast<float>(ub[s]) * tb[8 + s]);
+      const float L1 = s + 1 == M - 1 ? cc * usc : tb[s + 1] * (static_cast<float>(ub[s + 1 < M - 1 ? s + 1 : 0]) * tb[9 + s]);
+      float p[3], q[3];
+      split3(L0 * ksf[s], p[0], p[1], p[2]);
+      split3(L1 * (s + 1 == M - 1 ? misc[2] : ksf[s + 1]), q[0], q[1], q[2]);
+#pragma unroll
+      for (int j = 0; j < 3; j++) lw[4 * j + (s >> 1)] = bf2(p[j], q[j]);
+    }
+    __syncwarp();
+    const float2 al2 = make_float2(tb[16], tb[16]);
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+      uint32_t A1[2], A2[2], A3[2];
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const uint32_t* l = Lp + (warp * 32 + 16 * x + 8 * r + g) * 12 + t;
+        A1[r] = l[0]; A2[r] = l[4]; A3[r] = l[8];
+      }
+      if constexpr (!QUANT) {
+#pragma unroll
+        for (int un = 0; un < NU; un++) {
+          const uint4 kf = *reinterpret_cast<const uint4*>(KBf + (un * 32 + lane) * 4);
+          const uint32_t kb[4] = {kf.x, kf.y, kf.z, kf.w};
+#pragma unroll
+          for (int p = 0; p < 4; p++) {                    // the two rows' words of one column pair
+            uint32_t &wa = sw[x][0][un * WPU + p], &wc = sw[x][1][un * WPU + p];
+            const float2 fa = __fmul2_rn(make_float2(__uint_as_float(wa << 16), __uint_as_float(wa & 0xFFFF0000u)), al2);
+            const float2 fc = __fmul2_rn(make_float2(__uint_as_float(wc << 16), __uint_as_float(wc & 0xFFFF0000u)), al2);
+            float acc[4] = {fa.x, fa.y, fc.x, fc.y};
+            mma_bf16(acc, A1[0], A1[1], A2[0], A2[1], kb[p], kb[p]);
+            mma_bf16_k8(acc, A3[0], A3[1], kb[p]);
+            wa = bf2(acc[0], acc[1]);
+            wc = bf2(acc[2], acc[3]);
+          }
+        }
+      } else {
+        auto halves = [&](auto nh, auto hc) {              // NH units from unit H0 on
+          constexpr int NH = decltype(nh)::value, H0 = decltype(hc)::value, NS = UPG == 1 ? NH : 1, G0 = H0 / UPG;
+          uint32_t m[NH][4], o[NH][4];
+          float sc[2][NS], acc[NH][4][4];
+#pragma unroll
+          for (int n = 0; n < NH; n++) {
+#pragma unroll
+            for (int p = 0; p < WPU; p++) { m[n][2 * p] = sw[x][0][(H0 + n) * WPU + p]; m[n][2 * p + 1] = sw[x][1][(H0 + n) * WPU + p]; }
+          }
+#pragma unroll
+          for (int i = 0; i < NS; i++) { sc[0][i] = h2f(scr[x][0][G0 + i]); sc[1][i] = h2f(scr[x][1][G0 + i]); }
+          fold_acc<BITS, UPG, NH, false>(m, sc, A1, A2, A3, KBf, H0, lane, al2, nullptr, acc);
+          const float s_own = fold_round<BITS, UPG, NH>(acc, lane, o);
+          if (NS == 2 || t < 2) SCrow[(16 * x + 8 * (t & 1)) * NG + G0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);
+#pragma unroll
+          for (int n = 0; n < NH; n++) {
+#pragma unroll
+            for (int p = 0; p < WPU; p++) { sw[x][0][(H0 + n) * WPU + p] = o[n][2 * p]; sw[x][1][(H0 + n) * WPU + p] = o[n][2 * p + 1]; }
+          }
+        };
+        halves(IntC<2>(), IntC<0>());
+        halves(IntC<NU - 2>(), IntC<2>());
+      }
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+#pragma unroll
+        for (int un = 0; un < NU; un++) st_words<WPU>(Srow + (16 * x + 8 * r) * ROWB + 4 * BITS * un, &sw[x][r][un * WPU]);
+      }
+    }
+  }
+}
+
+template <int KIND, int BITS, int DK, int DV, int HPS>
+int launch_reg_one(const StepArgs& a, cudaStream_t stream) {
+  StepArgs b = a;
+  b.gqa_full = a.HV / a.HK;
+  const dim3 grid(static_cast<unsigned>(a.rows), static_cast<unsigned>(a.HV / HPS));
+  // bf16 activations and output take the kernel with those element types compiled in
+  const bool bio = a.dt_qk == DT_BF16 && a.dt_v == DT_BF16 && a.dt_out == DT_BF16;
+  const cudaError_t e = bio ? launch_pdl(step_reg_kernel<KIND, BITS, DK, DV, HPS, true>, grid, HPS * DV, 0, stream, b)
+                            : launch_pdl(step_reg_kernel<KIND, BITS, DK, DV, HPS, false>, grid, HPS * DV, 0, stream, b);
+  return e == cudaSuccess ? 0 : -(1000 + static_cast<int>(e));
+}
+
+}  // namespace sqb

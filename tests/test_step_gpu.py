@@ -577,6 +577,39 @@ def test_long_tail_shapes_match_oracle(c, kernel_path):
     assert st['scal'] <= max(1, 1e-4 * st['ncodes']), st
 
 
+# the shapes of the register-tile step, and (last) one of its formats whose heads do not fill its CTAs
+REG_SHAPES = [
+    dict(kind='gdn', fmt='bf16', B=2, hv=4, hk=2, dk=128, dv=128, m=8, bb=8, seed=81),
+    dict(kind='gdn', fmt='bf16', B=1, hv=3, hk=1, dk=128, dv=128, m=8, bb=8, seed=82),
+    dict(kind='gdn', fmt='bf16', B=1, hv=8, hk=2, dk=128, dv=64, m=8, bb=8, seed=83),
+    dict(kind='m2', fmt='bf16', B=2, hv=8, hk=2, dk=128, dv=64, m=8, bb=8, seed=84),
+    dict(kind='m2', fmt='bf16', B=1, hv=2, hk=2, dk=128, dv=128, m=8, bb=8, seed=85),
+    dict(kind='gdn', fmt=(4, 'k', 64), B=2, hv=3, hk=3, dk=96, dv=192, m=8, bb=8, seed=86),
+    dict(kind='gdn', fmt=(8, 'k', 32), B=2, hv=3, hk=3, dk=96, dv=192, m=8, bb=8, seed=87),
+    dict(kind='gdn', fmt=(4, 'k', 64), B=1, hv=4, hk=2, dk=96, dv=128, m=8, bb=8, seed=88),
+    dict(kind='gdn', fmt=(8, 'k', 32), B=1, hv=4, hk=2, dk=96, dv=128, m=8, bb=8, seed=89),
+    dict(kind='gdn', fmt=(8, 'k', 32), B=1, hv=4, hk=1, dk=96, dv=64, m=8, bb=8, seed=90),
+    dict(kind='gdn', fmt='bf16', B=1, hv=3, hk=3, dk=128, dv=64, m=8, bb=8, seed=91),
+]
+
+
+@pytest.mark.parametrize('mode', ['fp32', 'bf16', 'extreme'])
+@pytest.mark.parametrize('c', REG_SHAPES, ids=lambda c: f"{c['kind']}-{c['fmt']}-{c['dk']}x{c['dv']}-{c['hv']}.{c['hk']}")
+def test_register_tile_step_matches_oracle(c, mode, kernel_path):
+    """Two fold periods in both activation types and with read-out vectors that are zero, tiny or huge; same bar as the
+    other cases (fp32 sums in another order: 2e-5 of the largest output; a bf16 output one unit in the last place)."""
+    st = _oracle_lockstep(dict(c, extreme=mode == 'extreme'), T=2 * c['m'] + 3,
+                          act_dtype=torch.bfloat16 if mode == 'bf16' else torch.float32)
+    print(f"\n[{c['kind']} {c['fmt']} {c['dk']}x{c['dv']} {mode}] worst {st['worst']:.2e}, buffer {st['buf']}/{st['nbuf']}, "
+          f"codes {st['codes']}/{st['ncodes']}, scales {st['scal']}")
+    assert st['worst'] < (1e-2 if mode == 'bf16' else 2e-5), st
+    # an fp16 scale that fell on the other side of a tie (the device's exp and log against the host's in Mamba2's softplus)
+    # moves x / scale by 2^-11 of it, at most 127 / 2048 = 6 % of a step, and with it that share of the entries' codes
+    assert st['buf'] <= max(1, 1e-4 * st['nbuf']) + 0.0625 * max(c['dk'], c['dv']) * st['scal'], st
+    assert st['codes'] <= max(1, 1e-4 * st['ncodes']), st
+    assert st['scal'] <= max(1, 1e-4 * st['ncodes']), st
+
+
 INT4V_128 = dict(kind='gdn', fmt=(4, 'v', 32), B=1, hv=4, hk=2, dk=128, dv=128, m=8, bb=8, T=17, seed=73)
 
 
