@@ -242,8 +242,10 @@ int64_t sqb_launch_count(void);
    (direct loads, folds inside its own launch; any supported shape); 2 the staged SIMT kernel (one CTA per batch row
    and key head, the state staged through shared memory by bulk async copies) followed by the fold launch; 3 the
    tensor-core kernel (the state pass as integer mma.sync products) followed by the fold launch; 4 the tensor-core
-   kernel with the fold of a slot's m-th token inside its launch (what 0 picks wherever the shape allows).  A path
-   that does not take a shape falls through to the next lower one.  "force_generic_kernel" = 1 is the same as
+   kernel with the fold of a slot's m-th token inside its launch (what 0 picks wherever the shape allows and the grid is
+   longer than one wave); 5 the register-tile kernel (the state loaded straight into matrix fragments; what 0 picks for
+   grids of one wave, and every path but 1 for the shapes that 3 and 4 do not take).  A path that does not take a shape
+   falls through to the next lower one.  "force_generic_kernel" = 1 is the same as
    kernel_path 1 (and sends every GGA head to the tile kernel).  The paths agree up to the order of fp32 sums.
    "wait_limit_us": how long a device-side wait for a bulk copy may last before the CTA gives up (default 1 s).
    "mma_heads_per_cta": value heads a CTA of the tensor-core kernels takes (0: the default, two stages of 128 rows).

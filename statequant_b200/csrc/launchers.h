@@ -39,17 +39,18 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, 
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
-// Shapes the register-tile step takes: bf16 states of d_k 128 and d_v 64 or 128; Gated DeltaNet states of d_k 96 and d_v 64,
-// 128 or 192 with 8-bit codes in key groups of 32 or 4-bit codes in key groups of 64; decays per head, int8 buffer of 8,
-// q / k per key head, a CTA's rows of one key head.  The rest (fp32 states, KDA, other dims) is the generic kernel's.
+// Shapes the register-tile step takes: d_k 128 and d_v 64 or 128 with bf16 states or (Gated DeltaNet, Mamba2) 8-bit codes in
+// key groups of 32 or 4-bit codes in key groups of 64; Gated DeltaNet states of d_k 96 and d_v 64, 128 or 192 with those codes;
+// decays per head, int8 buffer of 8, q / k per key head, a CTA's rows of one key head.
 inline bool reg_shape_ok(const StepArgs& a, int bits, bool axk, int kind) {
   if (kind == K_KDA || !a.qbuf || a.M != 8 || (!a.per_key_head && a.HV != a.HK)) return false;
-  if (bits == 16) {
-    if (a.DK != 128 || (a.DV != 64 && a.DV != 128)) return false;
-  } else {
-    if (kind != K_GDN || !axk || a.DK != 96 || (a.DV != 64 && a.DV != 128 && a.DV != 192)) return false;
-    if (!((bits == 8 && a.group == 32) || (bits == 4 && a.group == 64))) return false;
-  }
+  if (bits != 16 && !(axk && ((bits == 8 && a.group == 32) || (bits == 4 && a.group == 64)))) return false;
+  const bool wide = a.DK == 128 && (a.DV == 64 || a.DV == 128);
+  const bool odd = a.DK == 96 && bits != 16 && kind == K_GDN && (a.DV == 64 || a.DV == 128 || a.DV == 192);
+  if (!wide && !odd) return false;
+  // a row's scales are one 4- or 8-byte load where there are two or four of them
+  const int ng = bits == 16 ? 1 : a.DK == 96 ? (bits == 8 ? 1 : 2) : a.DK / a.group;
+  if ((reinterpret_cast<uintptr_t>(a.SC) | static_cast<uintptr_t>(a.sSC)) % (2 * ng)) return false;
   const int hps = a.DV == 64 ? 2 : 1;
   return (a.HV / a.HK) % hps == 0 && a.HV / hps <= 65535;
 }

@@ -63,11 +63,11 @@ __device__ __forceinline__ FxScale fx30_scale(float amax) {
   if (!(amax <= 3.0e38f)) { s.m1 = 0.f; s.m2 = 0.f; s.i1 = __uint_as_float(0x7FC00000u); }
   return s;
 }
-// the four balanced digits of x (|x| <= 2^30) as the bytes of the result, lowest digit in byte 0
-__device__ __forceinline__ uint32_t fx30_digits(float v, const FxScale& s) {
-  const int x = __float2int_rn((v * s.m1) * s.m2);
-  return (static_cast<uint32_t>(x) + 0x80808080u) ^ 0x80808080u;
+// the four balanced digits of x (|x| <= 2^30, rounded to an integer) as the bytes of the result, lowest digit in byte 0
+__device__ __forceinline__ uint32_t byte_digits(float x) {
+  return (static_cast<uint32_t>(__float2int_rn(x)) + 0x80808080u) ^ 0x80808080u;
 }
+__device__ __forceinline__ uint32_t fx30_digits(float v, const FxScale& s) { return byte_digits((v * s.m1) * s.m2); }
 
 // One lane's four consecutive columns (4 lane .. 4 lane + 3) of vector `vec` -> its words of the B fragments in
 // shared memory, Bf[(unit * 2 + reg) * 32 + n * 4 + t].  All 32 lanes call this together.

@@ -183,6 +183,18 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
   const sqb::StepArgs& a = a0;
   const int path = g_force_generic.load(std::memory_order_relaxed) ? 1 : g_kernel_path.load(std::memory_order_relaxed);
   constexpr bool kda = KIND == sqb::K_KDA;
+  // The register-tile kernel (step_reg.cuh): shapes the tensor-core kernel does not take, and grids that fit the GPU at once
+  // (its CTAs are resident four to an SM).  There the serial chain of a CTA is what counts: it spreads a row over twice as many
+  // warps (a head per CTA) and reads and folds without a detour through shared memory.  In longer grids its larger share of
+  // per-CTA work counts.  us per layer and token, tensor-core kernel -> this one, int8 k/32, 32 heads of 128 x 128, slots
+  // folding together / each on a token of its own: 1 row 4.9 -> 3.2 / 4.9 -> 3.2, 8 rows 5.2 -> 3.9 / 10.0 -> 6.0, 16 rows (512
+  // CTAs) 5.9 -> 5.6 / 11.6 -> 7.8, 24 rows 8.2 -> 8.7 / 16.2 -> 10.8, 256 rows 44.9 -> 60.2 / 57.9 -> 63.3.
+  constexpr long long ONE_WAVE = 4 * 148;
+  if (path != 1 && sqb::reg_shape_ok(a0, bits, axk, KIND)) {
+    const bool few = static_cast<long long>(a0.rows) * (a0.HV / (a0.DV == 64 ? 2 : 1)) <= ONE_WAVE;
+    if (path == 5 || (path == 0 && few) || !sqb::mma_shape_ok(a0, bits, axk, kda, KIND))
+      return sub_rc(sqb::launch_reg(KIND, a0, bits, stream));
+  }
   // Every check that could refuse a launch is made before the first one: a positive "shape not taken" code after a
   // step kernel has appended would leave the slot between two states.
   if ((path == 0 || path >= 3) && sqb::mma_shape_ok(a0, bits, axk, kda, KIND)) {
@@ -203,7 +215,6 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
       return rf <= 0 ? rf : fail(SQB_ECUDA, "fold kernel refused a checked shape");
     }
   }
-  if (path != 1 && sqb::reg_shape_ok(a, bits, axk, KIND)) return sub_rc(sqb::launch_reg(KIND, a, bits, stream));
   if (path != 1 && tma_ok(a, bits, axk, kda) && fold_fits(a, bits, axk, kda)) {
     // the staged kernel only appends on a slot's m-th token; the fold launch that follows it rewrites the state of
     // the heads whose buffer is full (the generic kernel folds inside its own launch)
@@ -238,7 +249,7 @@ int64_t sqb_launch_count(void) { return g_launches.load(); }
 
 int sqb_set_option(const char* name, int value) {
   if (name && !strcmp(name, "force_generic_kernel")) { g_force_generic = value; return 0; }
-  if (name && !strcmp(name, "kernel_path") && value >= 0 && value <= 4) { g_kernel_path = value; return 0; }
+  if (name && !strcmp(name, "kernel_path") && value >= 0 && value <= 5) { g_kernel_path = value; return 0; }
   if (name && !strcmp(name, "mma_heads_per_cta") && value >= 0) { g_mma_hpc = value; return 0; }
   if (name && !strcmp(name, "wait_limit_us") && value > 0) { g_wait_ns = 1000ll * value; return 0; }
   if (name && !strcmp(name, "test_extra_tx") && value >= 0 && value % 16 == 0) { g_test_extra_tx = value; return 0; }

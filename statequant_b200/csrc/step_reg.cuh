@@ -1,6 +1,6 @@
-// The fused decode step with the state held in REGISTERS: bf16 states of d_k 128, and 4- / 8-bit states of d_k 96 scaled along
-// k (groups of 64 / 32, the last one short); decays per head (Gated DeltaNet; bf16: Mamba2 too), int8 buffer of 8, q / k per
-// key head.
+// The fused decode step with the state held in REGISTERS: bf16 states of d_k 128, and 4- / 8-bit states of d_k 128 or 96 scaled
+// along k (groups of 64 / 32, the last one of 96 columns short); decays per head (Gated DeltaNet, Mamba2), int8 buffer of 8,
+// q / k per key head.
 //
 // One CTA per (batch row, ROWS state rows), a thread per row: one head of d_v 128 or 192, two heads of d_v 64 (of one key
 // head).  Warp w owns rows 32 w .. 32 w + 31 = two blocks of 16; lane (g, t) = (lane / 4, lane % 4) loads rows g and g + 8 of
@@ -11,15 +11,16 @@
 // came into.
 //
 // Read-out, bf16: q and k are cut into three bf16 pieces each (8 + 8 + 8 mantissa bits: exact), the columns of B; every
-// product is exact and a unit of 32 columns is summed from zero by the tensor core, the units in fp32.  Columns 0, 1, 2 are
+// product is exact; 16 columns at a time are summed from zero by the tensor core, the eight sums in an fp32 tree.  Columns 0, 1, 2 are
 // the pieces of q, 4, 5, 6 those of k, so that the thread pair t = 0, 1 holds the parts of q and t = 2, 3 those of k.
 // Integer states: the byte digits of mma_pass.cuh, exact integer sums.
 // Fold: fold_mma.cuh's (three bf16 pieces of L against the int8 key codes), accumulators started at decay * state.
 //
-// HBM-bound by intent: a CTA's whole state is in flight at once.  Measured per layer and token, generic kernel -> this one
-// (the generic kernel's CTA goes through six block reductions before its state pass and holds 12 warps per SM): bf16, 96 rows
-// of 32 heads of 128 x 128, 120 -> 31.6 us (18 us at the copy rate); 4-bit, 64 rows of 30 heads of 96 x 192, a slot in eight
-// folding, 103 -> 26.6 us.
+// HBM-bound by intent (a CTA's whole state is in flight at once); small grids are bound by the serial chain idx -> state and
+// prologue -> read-out -> append, which is why q and k are taken as they come and their norms applied to the finished sums.
+// Measured per layer and token, generic kernel -> this one (the generic kernel's CTA goes through six block reductions before
+// its state pass and holds 12 warps per SM): bf16, 96 rows of 32 heads of 128 x 128, 120 -> 29.6 us (18 us at the copy rate);
+// 4-bit, 64 rows of 30 heads of 96 x 192, a slot in eight folding, 103 -> 25.2 us.  Against the tensor-core kernel: sqb200.cu.
 #pragma once
 #include "launchers.h"
 #include "step_tma.cuh"
@@ -27,8 +28,10 @@
 
 namespace sqb {
 
-// CTAs per SM: bf16 holds 64 words of state per thread (128 registers), integer states 12 to 32 (80 registers)
-constexpr int reg_min_ctas(int bits, int threads) { return (bits == 16 ? 512 : 768) / threads; }
+// Threads per SM: bf16 holds 64 words of state per thread (128 registers); integer states of d_k 128 come here in grids of up
+// to four CTAs per SM, and need the registers more than the residency; those of d_k 96 in grids of any size (80 registers:
+// 852 us a pass against 955 us with 112).
+constexpr int reg_min_ctas(int bits, int dk, int threads) { return (bits == 16 || dk == 128 ? 512 : 768) / threads; }
 
 // N words of a lane's slice of a unit: 4 (bf16), 2 (int8) or 1 (int4)
 template <int N>
@@ -43,6 +46,19 @@ __device__ __forceinline__ void st_words(uint8_t* p, const uint32_t* r) {
   else if constexpr (N == 2) *reinterpret_cast<uint2*>(p) = make_uint2(r[0], r[1]);
   else *reinterpret_cast<uint32_t*>(p) = r[0];
 }
+
+// the NG scales of a row as packed words: one load where the row's scales are an aligned 4 or 8 bytes
+template <int NG>
+__device__ __forceinline__ void ld_scales(uint32_t* r, const unsigned short* p) {
+  if constexpr (NG == 4) { const uint2 v = *reinterpret_cast<const uint2*>(p); r[0] = v.x; r[1] = v.y; }
+  else if constexpr (NG == 2) r[0] = *reinterpret_cast<const uint32_t*>(p);
+  else {
+    r[0] = p[0];
+    if constexpr (NG > 1) r[0] |= static_cast<uint32_t>(p[1]) << 16;
+    if constexpr (NG > 2) r[1] = p[2];
+  }
+}
+__device__ __forceinline__ float scale_of(const uint32_t* r, int i) { return h2f(static_cast<unsigned short>(r[i >> 1] >> (16 * (i & 1)))); }
 
 // The gates of value head h (one lane per head calls it): g, beta | dt, gcur, exp(gcur), exp(g), gcur + g, D into o[0 .. 6].
 // In two steps, so that the loads of a warp are in flight before their first use.
@@ -96,7 +112,7 @@ __device__ __forceinline__ void gates_finish(const StepArgs& A, const GateRaw& w
 __device__ __forceinline__ float add_parts(float hi, float lo) { return fabsf(hi) <= 3.402823466e38f ? hi + lo : hi; }
 
 template <int KIND, int BITS, int DK, int DV, int HPS, bool BIO>
-__global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_reg_kernel(const __grid_constant__ StepArgs A) {
+__global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) step_reg_kernel(const __grid_constant__ StepArgs A) {
   dependency_wait();
   dependency_release();
   constexpr int NT = HPS * DV, M = 8, WPH = DV / 32, NU = DK / 32, CW = 4, ROWB = DK * BITS / 8;
@@ -111,7 +127,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
   __shared__ __align__(16) int8_t kcur[DK];
   __shared__ __align__(16) float hd[HPS * HD_W];
   __shared__ float2 dcu[HPS * M], dqk[M];
-  __shared__ float gbs[HPS * M], ksf[M], tab[HPS * 20], red[NT / 32], misc[8];
+  __shared__ float gbs[HPS * M], ksf[M], tab[HPS * 20], red[NT / 32], misc[12];
 
   const int dt_qk = BIO ? static_cast<int>(DT_BF16) : A.dt_qk, dt_v = BIO ? static_cast<int>(DT_BF16) : A.dt_v,
             dt_out = BIO ? static_cast<int>(DT_BF16) : A.dt_out;
@@ -169,7 +185,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
   const long long row0 = (long long)h * DV + rv0 + g;      // row g of the warp's first block
   uint8_t* Srow = A.S + seq * A.sS + row0 * ROWB + BITS * t;
   uint32_t sw[2][2][NU * WPU];                             // [block][row g, row g + 8][unit, word]
-  unsigned short scr[2][2][NG];
+  uint32_t scr[2][2][(NG + 1) / 2];                        // their scales, two to a word
   unsigned short* SCrow = nullptr;
   if (QUANT) SCrow = reinterpret_cast<unsigned short*>(A.SC + seq * A.sSC) + row0 * NG;
 #pragma unroll
@@ -179,8 +195,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
 #pragma unroll
       for (int u = 0; u < NU; u++) ld_words<WPU>(&sw[x][r][u * WPU], Srow + (16 * x + 8 * r) * ROWB + 4 * BITS * u);
       if constexpr (QUANT) {
-#pragma unroll
-        for (int i = 0; i < NG; i++) scr[x][r][i] = SCrow[(16 * x + 8 * r) * NG + i];
+        ld_scales<NG>(scr[x][r], SCrow + (16 * x + 8 * r) * NG);
       }
     }
   }
@@ -194,18 +209,22 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
   uint32_t kword = 0;                                      // warp 3: the key as it goes into the buffer
   float kscale = 0.f;
   if (warp == 0) {
+    // q and k as they come, scaled by powers of two (30-bit fixed point, mma_pass.cuh); what their norms make of the
+    // results, warp 3 finds out meanwhile and every row applies at the end
     float qr[CW], kr[CW];
     cvt4_raw(rq, dt_qk, qr);
     cvt4_raw(rk, dt_qk, kr);
-    if (KIND != K_M2) {
-      float s0 = 0.f, s1 = 0.f;
+    float d = 0.f, mq = 0.f, mk = 0.f;
 #pragma unroll
-      for (int j = 0; j < CW; j++) { s0 += qr[j] * qr[j]; s1 += kr[j] * kr[j]; }
-      s0 = warp_sum(s0);
-      s1 = warp_sum(s1);
-      const float nq = __fsqrt_rn(s0 + 1e-6f), nk = __fsqrt_rn(s1 + 1e-6f);
+    for (int j = 0; j < CW; j++) { mq = fmaxf(mq, fabsf(qr[j])); mk = fmaxf(mk, fabsf(kr[j])); }
+    mq = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mq)));
+    mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
+    const FxScale fq = fx30_scale(mq), fk = fx30_scale(mk);
 #pragma unroll
-      for (int j = 0; j < CW; j++) { qr[j] = __fdiv_rn(qr[j], nq) * A.scale; kr[j] = __fdiv_rn(kr[j], nk); }
+    for (int j = 0; j < CW; j++) {
+      qr[j] = (qr[j] * fq.m1) * fq.m2;
+      kr[j] = (kr[j] * fk.m1) * fk.m2;
+      d += kr[j] * qr[j];
     }
     // bf16: the state pass's fragments: lane l's columns 4 l .. 4 l + 3 are step l / 8 * 2 + l % 2, thread (l % 8) / 2
     if constexpr (!QUANT) {
@@ -222,21 +241,11 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
       }
     }
     // the buffered keys against q and k: integer digits (mma_pass.cuh), the key codes straight from the loads
-    float d = 0.f, mq = 0.f, mk = 0.f;
-#pragma unroll
-    for (int j = 0; j < CW; j++) {
-      d += kr[j] * qr[j];
-      mq = fmaxf(mq, fabsf(qr[j]));
-      mk = fmaxf(mk, fabsf(kr[j]));
-    }
-    mq = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mq)));
-    if (TWO) mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
-    const FxScale fq = fx30_scale(mq), fk = fx30_scale(mk);
 #pragma unroll
     for (int vec = 0; vec < 2; vec++) {
       uint32_t y[CW];
 #pragma unroll
-      for (int j = 0; j < CW; j++) y[j] = vec == 0 ? fx30_digits(qr[j], fq) : (TWO ? fx30_digits(kr[j], fk) : 0u);
+      for (int j = 0; j < CW; j++) y[j] = vec == 0 ? byte_digits(qr[j]) : (TWO ? byte_digits(kr[j]) : 0u);
       const uint32_t t0 = __byte_perm(y[0], y[1], 0x5140), t1 = __byte_perm(y[2], y[3], 0x5140);
       const uint32_t t2 = __byte_perm(y[0], y[1], 0x7362), t3 = __byte_perm(y[2], y[3], 0x7362);
       const uint32_t W[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410),
@@ -257,7 +266,6 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
     const float wa = (t & 1) ? 256.0f : 16777216.0f, wb = (t & 1) ? 1.0f : 65536.0f;
     float T = fmaf((__int_as_float(acc[0]) - 12582912.0f) * ksl, wa, ((__int_as_float(acc[1]) - 12582912.0f) * ksl) * wb);
     T += __shfl_xor_sync(0xffffffffu, T, 1);
-    T = t < 2 ? (T * fq.i1) * fq.i2 : (T * fk.i1) * fk.i2;
     if (t == 0) { dqk[g].x = T; ksf[g] = ksl; }
     if (t == 2) dqk[g].y = T;
   } else if (warp == 1) {
@@ -271,15 +279,18 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
       gbs[lane] = gb0;
     }
   } else if (warp == 3) {
-    // the key, rounded: its normalisation is redone here (the arithmetic of warp 0, so the same bits)
+    // the norms, and the key as it goes into the buffer
     float kr[CW];
     cvt4_raw(rk, dt_qk, kr);
     if (KIND != K_M2) {
-      float s1 = 0.f;
+      float qr[CW], s0 = 0.f, s1 = 0.f;
+      cvt4_raw(rq, dt_qk, qr);
 #pragma unroll
-      for (int j = 0; j < CW; j++) s1 += kr[j] * kr[j];
+      for (int j = 0; j < CW; j++) { s0 += qr[j] * qr[j]; s1 += kr[j] * kr[j]; }
+      s0 = warp_sum(s0);
       s1 = warp_sum(s1);
       const float nk = __fsqrt_rn(s1 + 1e-6f);
+      if (lane == 0) { misc[8] = __fdiv_rn(A.scale, __fsqrt_rn(s0 + 1e-6f)); misc[9] = __fdiv_rn(1.0f, nk); }
 #pragma unroll
       for (int j = 0; j < CW; j++) kr[j] = __fdiv_rn(kr[j], nk);
     }
@@ -294,7 +305,10 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
     if (lane == 0) misc[2] = kscale;
   }
   __syncthreads();
-  const float kq = misc[0];
+  // back from fixed point and, but for Mamba2, over the norm: powers of two (exact) and one factor per vector
+  const float iq1 = misc[4], iq2 = KIND == K_M2 ? misc[5] : misc[5] * misc[8];
+  const float ik1 = misc[6], ik2 = KIND == K_M2 ? misc[7] : misc[7] * misc[9];
+  const float kq = (((misc[0] * iq1) * iq2) * ik1) * ik2;
   const int n0 = __float_as_int(misc[1]);                  // live buffer entries of this slot
   const bool full = n0 == M - 1;                           // this token fills the buffer: fold after the read-out
   if (warp == 3 && first) {
@@ -307,19 +321,24 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
   if constexpr (!QUANT) {
 #pragma unroll
     for (int x = 0; x < 2; x++) {
-      float2 s01 = make_float2(0.f, 0.f), s23 = s01;
+      float2 s01[NU], s23[NU];
 #pragma unroll
       for (int u = 0; u < NU; u++) {
         const uint2 b0 = Bf[(2 * u) * 32 + lane], b1 = Bf[(2 * u + 1) * 32 + lane];
         const uint32_t *wa = &sw[x][0][u * WPU], *wc = &sw[x][1][u * WPU];
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_bf16(acc, wa[0], wc[0], wa[1], wc[1], b0.x, b0.y);
-        mma_bf16(acc, wa[2], wc[2], wa[3], wc[3], b1.x, b1.y);
-        s01 = __fadd2_rn(s01, make_float2(acc[0], acc[1]));
-        s23 = __fadd2_rn(s23, make_float2(acc[2], acc[3]));
+        float e[4] = {0.f, 0.f, 0.f, 0.f}, f[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16(e, wa[0], wc[0], wa[1], wc[1], b0.x, b0.y);
+        mma_bf16(f, wa[2], wc[2], wa[3], wc[3], b1.x, b1.y);
+        s01[u] = __fadd2_rn(make_float2(e[0], e[1]), make_float2(f[0], f[1]));
+        s23[u] = __fadd2_rn(make_float2(e[2], e[3]), make_float2(f[2], f[3]));
+      }
+#pragma unroll
+      for (int n = NU / 2; n > 0; n >>= 1) {
+#pragma unroll
+        for (int u = 0; u < n; u++) { s01[u] = __fadd2_rn(s01[u], s01[u + n]); s23[u] = __fadd2_rn(s23[u], s23[u + n]); }
       }
       // t even: (hi, mid); t odd: (lo, -).  The even lane of a pair ends up with row g, the odd one with row g + 8.
-      const float v0 = (t & 1) ? s01.x : add_parts(s01.x, s01.y), v1 = (t & 1) ? s23.x : add_parts(s23.x, s23.y);
+      const float v0 = (t & 1) ? s01[0].x : add_parts(s01[0].x, s01[0].y), v1 = (t & 1) ? s23[0].x : add_parts(s23[0].x, s23[0].y);
       const float own = (t & 1) ? v1 : v0, recv = __shfl_xor_sync(0xffffffffu, (t & 1) ? v0 : v1, 1);
       y[x] = (t & 1) ? add_parts(recv, own) : add_parts(own, recv);
     }
@@ -339,7 +358,6 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
       ci[i][0] = MAGIC_I - 8 * d[0];
       ci[i][1] = MAGIC_I - 8 * d[1];
     }
-    const float i1 = t < 2 ? misc[4] : misc[6], i2 = t < 2 ? misc[5] : misc[7];
 #pragma unroll
     for (int x = 0; x < 2; x++) {
       float2 p01 = make_float2(0.f, 0.f), p23 = p01;
@@ -355,13 +373,13 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
             mma_i8<true>(acc, wa[0] & 0x0F0F0F0Fu, wc[0] & 0x0F0F0F0Fu, (wa[0] >> 4) & 0x0F0F0F0Fu, (wc[0] >> 4) & 0x0F0F0F0Fu,
                          bf[2 * u], bf[2 * u + 1]);
         }
-        const float sa = h2f(scr[x][0][i]), sc = h2f(scr[x][1][i]);
+        const float sa = scale_of(scr[x][0], i), sc = scale_of(scr[x][1], i);
         const float2 nm = make_float2(-12582912.0f, -12582912.0f);
         p01 = __ffma2_rn(__fadd2_rn(make_float2(__int_as_float(acc[0]), __int_as_float(acc[1])), nm), make_float2(sa, sa), p01);
         p23 = __ffma2_rn(__fadd2_rn(make_float2(__int_as_float(acc[2]), __int_as_float(acc[3])), nm), make_float2(sc, sc), p23);
       }
       const float p[4] = {p01.x, p01.y, p23.x, p23.y};
-      y[x] = (join_digits(p, t) * i1) * i2;                // powers of two: exact
+      y[x] = join_digits(p, t);
     }
   }
   float tq, tk;
@@ -383,6 +401,8 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
       if (TWO) tk = fmaf(xb, du.x * dd.y, tk);
     }
   }
+  tq = (tq * iq1) * iq2;
+  tk = (tk * ik1) * ik2;
   float u, o;
   if (KIND == K_GDN) {
     u = hda.y * fmaf(-hdb.x, tk, vt);
@@ -477,7 +497,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, HPS * DV)) step_r
             for (int p = 0; p < WPU; p++) { m[n][2 * p] = sw[x][0][(H0 + n) * WPU + p]; m[n][2 * p + 1] = sw[x][1][(H0 + n) * WPU + p]; }
           }
 #pragma unroll
-          for (int i = 0; i < NS; i++) { sc[0][i] = h2f(scr[x][0][G0 + i]); sc[1][i] = h2f(scr[x][1][G0 + i]); }
+          for (int i = 0; i < NS; i++) { sc[0][i] = scale_of(scr[x][0], G0 + i); sc[1][i] = scale_of(scr[x][1], G0 + i); }
           fold_acc<BITS, UPG, NH, false>(m, sc, A1, A2, A3, KBf, H0, lane, al2, nullptr, acc);
           const float s_own = fold_round<BITS, UPG, NH>(acc, lane, o);
           if (NS == 2 || t < 2) SCrow[(16 * x + 8 * (t & 1)) * NG + G0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);

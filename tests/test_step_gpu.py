@@ -589,13 +589,18 @@ REG_SHAPES = [
     dict(kind='gdn', fmt=(4, 'k', 64), B=1, hv=4, hk=2, dk=96, dv=128, m=8, bb=8, seed=88),
     dict(kind='gdn', fmt=(8, 'k', 32), B=1, hv=4, hk=2, dk=96, dv=128, m=8, bb=8, seed=89),
     dict(kind='gdn', fmt=(8, 'k', 32), B=1, hv=4, hk=1, dk=96, dv=64, m=8, bb=8, seed=90),
+    dict(kind='gdn', fmt=(8, 'k', 32), B=2, hv=4, hk=2, dk=128, dv=128, m=8, bb=8, seed=92),
+    dict(kind='gdn', fmt=(4, 'k', 64), B=1, hv=3, hk=1, dk=128, dv=128, m=8, bb=8, seed=93),
+    dict(kind='gdn', fmt=(8, 'k', 32), B=1, hv=4, hk=2, dk=128, dv=64, m=8, bb=8, seed=94),
+    dict(kind='m2', fmt=(8, 'k', 32), B=2, hv=8, hk=2, dk=128, dv=64, m=8, bb=8, seed=95),
+    dict(kind='m2', fmt=(4, 'k', 64), B=1, hv=2, hk=2, dk=128, dv=128, m=8, bb=8, seed=96),
     dict(kind='gdn', fmt='bf16', B=1, hv=3, hk=3, dk=128, dv=64, m=8, bb=8, seed=91),
 ]
 
 
 @pytest.mark.parametrize('mode', ['fp32', 'bf16', 'extreme'])
 @pytest.mark.parametrize('c', REG_SHAPES, ids=lambda c: f"{c['kind']}-{c['fmt']}-{c['dk']}x{c['dv']}-{c['hv']}.{c['hk']}")
-def test_register_tile_step_matches_oracle(c, mode, kernel_path):
+def test_register_tile_step_matches_oracle(c, mode):
     """Two fold periods in both activation types and with read-out vectors that are zero, tiny or huge; same bar as the
     other cases (fp32 sums in another order: 2e-5 of the largest output; a bf16 output one unit in the last place)."""
     st = _oracle_lockstep(dict(c, extreme=mode == 'extreme'), T=2 * c['m'] + 3,
