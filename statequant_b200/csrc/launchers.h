@@ -23,6 +23,16 @@ struct SmemLimit {
     return e;
   }
 };
+// Launch in plain stream order: the grid's CTAs enter once the kernel in front of it has finished.
+template <class... P, class... A>
+cudaError_t launch_plain(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 // Launch with programmatic stream serialisation: the grid's CTAs may be scheduled before the kernel in front of it has
 // finished; the kernel itself waits for that (dependency_wait in common.cuh) before it touches memory.
 template <class... P, class... A>
