@@ -346,8 +346,7 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
   const int hh = (g * R) / DV;                         // head of this thread's rows within the stage
   const float* tb = tab + hh * TABW;
   const float2 al2 = make_float2(tb[16], tb[16]);
-#pragma unroll 1
-  for (int bb = 0; bb < 2; bb++) {
+  auto block = [&](int bb) {
     const int b = 2 * w + bb;
     const int row0 = g * R + 2 * b;                    // stage rows row0, row0 + 1
     uint32_t A1[2], A2[2], A3[2];
@@ -407,9 +406,22 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
         stsm_x2(addr, o[0][0], o[0][1]);
       }
     };
+    if constexpr (READ && BITS == 4) {
+#pragma unroll
+      for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
+    } else {
 #pragma unroll 1
-    for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
+      for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
+    }
     if constexpr (NHALF % 2 == 1) chunk(IntC<1>(), NHALF - 1);
+  };
+  // (the 4-bit read-out unrolled: 82 rows of 16 heads 30.4 -> 29.4 us; 8-bit, 256 rows: 121.9 as a loop, 123.5 unrolled)
+  if constexpr (READ && BITS == 4) {
+#pragma unroll
+    for (int bb = 0; bb < 2; bb++) block(bb);
+  } else {
+#pragma unroll 1
+    for (int bb = 0; bb < 2; bb++) block(bb);
   }
 }
 
