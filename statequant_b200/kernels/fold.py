@@ -14,7 +14,6 @@ from .formats import (check_dims, l2norm, pack, pack_vk, packed_format, pow2, st
                       unpack_vk)
 from .layout import set_shape
 from .lockstep import LockstepTables
-from .slots import _gdn_inputs
 
 
 class PackedGDNState(LockstepTables):
@@ -53,8 +52,16 @@ class PackedGDNState(LockstepTables):
         for t in (q, k, v, g, beta):
             assert t.is_contiguous()
         hq = HK if per_key else HV
-        a = _gdn_inputs(None, q.view(B, hq, DK), k.view(B, hq, DK), v.view(B, HV, DV), self.O.view(B, HV, DV), scale,
-                        g.view(B, HV), beta.view(B, HV), None, per_key)
+        assert k.dtype == q.dtype and g.dtype == beta.dtype
+        if not (q.numel() == k.numel() == B * hq * DK and v.numel() == B * HV * DV and g.numel() == beta.numel() == B * HV):
+            raise RuntimeError(f'step: q, k [{B * hq}, {DK}], v [{B * HV}, {DV}] and g, beta [{B * HV}] expected, got '
+                               f'{[tuple(t.shape) for t in (q, k, v, g, beta)]}')
+        # sqb_gdn_inputs_t in its field order; the tensors are dense, so a row's stride is its size
+        code, O = _cabi.dtype_code, self.O
+        sq, sv, sg = hq * DK * q.element_size(), HV * DV * v.element_size(), HV * g.element_size()
+        a = _cabi.GdnInputs(None, q.data_ptr(), sq, k.data_ptr(), sq, v.data_ptr(), sv, g.data_ptr(), sg, beta.data_ptr(), sg,
+                            None, 0, None, 0, None, None, O.data_ptr(), HV * DV * O.element_size(), float(scale), B, int(per_key),
+                            0, code(q), code(v), code(g), 0, 0, 0, code(O), 0)
         _cabi.check(_cabi.lib().sqb_gdn_step(_cabi.C.byref(self._st), _cabi.C.byref(a),
                                              _cabi.current_stream(q.device)), 'sqb_gdn_step')
         return self.O
