@@ -47,13 +47,15 @@ __device__ __forceinline__ void mma_i8(int (&d)[4], uint32_t a0, uint32_t a1, ui
 }
 
 // ---- fixed point ----------------------------------------------------------------------------------------------------
-// Multipliers m1 m2 = 2^(29 - e) (e: exponent of the vector's largest magnitude) as two factors that are both normal
-// floats over the whole float range, and their inverses.  A non-finite amax poisons the inverse (outputs become NaN).
+// Multipliers m1 m2 = 2^(TOP - e) (e: exponent of the vector's largest magnitude, which lands in [2^TOP, 2^(TOP + 1))) as two
+// factors that are both normal floats over the whole float range, and their inverses.  A non-finite amax poisons the
+// inverse (outputs become NaN).
 struct FxScale { float m1, m2, i1, i2; };
-__device__ __forceinline__ FxScale fx30_scale(float amax) {
+template <int TOP>
+__device__ __forceinline__ FxScale fx_scale(float amax) {
   int e = static_cast<int>((__float_as_uint(amax) >> 23) & 0xFFu) - 127;
   e = max(e, -126);
-  const int sh = 29 - e;
+  const int sh = TOP - e;
   const int h2 = sh >> 1, h1 = sh - h2;
   FxScale s;
   s.m1 = __uint_as_float(static_cast<uint32_t>(127 + h1) << 23);
@@ -63,6 +65,7 @@ __device__ __forceinline__ FxScale fx30_scale(float amax) {
   if (!(amax <= 3.0e38f)) { s.m1 = 0.f; s.m2 = 0.f; s.i1 = __uint_as_float(0x7FC00000u); }
   return s;
 }
+__device__ __forceinline__ FxScale fx30_scale(float amax) { return fx_scale<29>(amax); }
 // the four balanced digits of x (|x| <= 2^30, rounded to an integer) as the bytes of the result, lowest digit in byte 0
 __device__ __forceinline__ uint32_t byte_digits(float x) {
   return (static_cast<uint32_t>(__float2int_rn(x)) + 0x80808080u) ^ 0x80808080u;

@@ -12,7 +12,8 @@
 //
 // Read-out, bf16: q and k are cut into three bf16 pieces each (8 + 8 + 8 mantissa bits: exact), the columns of B; every
 // product is exact; 16 columns at a time are summed from zero by the tensor core, the eight sums in an fp32 tree.  Columns 0, 1, 2 are
-// the pieces of q, 4, 5, 6 those of k, so that the thread pair t = 0, 1 holds the parts of q and t = 2, 3 those of k.
+// the pieces of q, 4, 5, 6 those of k, so that the thread pair t = 0, 1 holds the parts of q and t = 2, 3 those of k.  The vectors
+// are scaled below 2^-15 for this, so that 128 products with states up to the format's maximum do not overflow.
 // Integer states: the byte digits of mma_pass.cuh, exact integer sums.
 // Fold: fold_mma.cuh's (three bf16 pieces of L against the int8 key codes), accumulators started at decay * state.
 //
@@ -118,6 +119,8 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   constexpr int NT = HPS * DV, M = 8, WPH = DV / 32, NU = DK / 32, CW = 4, ROWB = DK * BITS / 8;
   constexpr int WPU = BITS / 4, UPG = BITS == 4 ? 2 : 1, NG = BITS == 16 ? 1 : (NU + UPG - 1) / UPG;
   constexpr bool TWO = KIND != K_M2, QUANT = BITS != 16;
+  constexpr int TOP = QUANT ? 29 : -16;                    // q and k lie below 2^(TOP + 1); the byte digits want 2^30
+  constexpr float UPF = QUANT ? 1.0f : 35184372088832.0f;  // 2^(29 - TOP)
   __shared__ __align__(16) uint2 Bf[QUANT ? 1 : 2 * NU * 32];          // bf16: B fragments of the state pass (bf16 pieces)
   __shared__ __align__(16) uint32_t Bf8[2 * 4 * 32];       // B fragments of byte codes (byte digits): key tile, int8 state
   __shared__ __align__(16) uint32_t Bf4[BITS == 4 ? 2 * 4 * 32 : 1];   // B fragments of nibble codes
@@ -209,8 +212,8 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   uint32_t kword = 0;                                      // warp 3: the key as it goes into the buffer
   float kscale = 0.f;
   if (warp == 0) {
-    // q and k as they come, scaled by powers of two (30-bit fixed point, mma_pass.cuh); what their norms make of the
-    // results, warp 3 finds out meanwhile and every row applies at the end
+    // q and k as they come, scaled by powers of two (integer states: 30-bit fixed point, mma_pass.cuh); what their norms make
+    // of the results, warp 3 finds out meanwhile and every row applies at the end
     float qr[CW], kr[CW];
     cvt4_raw(rq, dt_qk, qr);
     cvt4_raw(rk, dt_qk, kr);
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     for (int j = 0; j < CW; j++) { mq = fmaxf(mq, fabsf(qr[j])); mk = fmaxf(mk, fabsf(kr[j])); }
     mq = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mq)));
     mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
-    const FxScale fq = fx30_scale(mq), fk = fx30_scale(mk);
+    const FxScale fq = fx_scale<TOP>(mq), fk = fx_scale<TOP>(mk);
 #pragma unroll
     for (int j = 0; j < CW; j++) {
       qr[j] = (qr[j] * fq.m1) * fq.m2;
@@ -245,7 +248,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     for (int vec = 0; vec < 2; vec++) {
       uint32_t y[CW];
 #pragma unroll
-      for (int j = 0; j < CW; j++) y[j] = vec == 0 ? byte_digits(qr[j]) : (TWO ? byte_digits(kr[j]) : 0u);
+      for (int j = 0; j < CW; j++) y[j] = vec == 0 ? byte_digits(qr[j] * UPF) : (TWO ? byte_digits(kr[j] * UPF) : 0u);
       const uint32_t t0 = __byte_perm(y[0], y[1], 0x5140), t1 = __byte_perm(y[2], y[3], 0x5140);
       const uint32_t t2 = __byte_perm(y[0], y[1], 0x7362), t3 = __byte_perm(y[2], y[3], 0x7362);
       const uint32_t W[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410),
@@ -266,6 +269,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     const float wa = (t & 1) ? 256.0f : 16777216.0f, wb = (t & 1) ? 1.0f : 65536.0f;
     float T = fmaf((__int_as_float(acc[0]) - 12582912.0f) * ksl, wa, ((__int_as_float(acc[1]) - 12582912.0f) * ksl) * wb);
     T += __shfl_xor_sync(0xffffffffu, T, 1);
+    T *= 1.0f / UPF;                                       // (in the unit of the state's sums)
     if (t == 0) { dqk[g].x = T; ksf[g] = ksl; }
     if (t == 2) dqk[g].y = T;
   } else if (warp == 1) {
@@ -305,9 +309,10 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     if (lane == 0) misc[2] = kscale;
   }
   __syncthreads();
-  // back from fixed point and, but for Mamba2, over the norm: powers of two (exact) and one factor per vector
-  const float iq1 = misc[4], iq2 = KIND == K_M2 ? misc[5] : misc[5] * misc[8];
-  const float ik1 = misc[6], ik2 = KIND == K_M2 ? misc[7] : misc[7] * misc[9];
+  // back to the vectors' own size and, but for Mamba2, over the norm: powers of two (exact) and one factor per vector (with the
+  // first power, so that no step between lies beyond the sum and the result: states near the largest float)
+  const float iq1 = KIND == K_M2 ? misc[4] : misc[4] * misc[8], iq2 = misc[5];
+  const float ik1 = KIND == K_M2 ? misc[6] : misc[6] * misc[9], ik2 = misc[7];
   const float kq = (((misc[0] * iq1) * iq2) * ik1) * ik2;
   const int n0 = __float_as_int(misc[1]);                  // live buffer entries of this slot
   const bool full = n0 == M - 1;                           // this token fills the buffer: fold after the read-out

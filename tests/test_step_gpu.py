@@ -615,6 +615,44 @@ def test_register_tile_step_matches_oracle(c, mode):
     assert st['scal'] <= max(1, 1e-4 * st['ncodes']), st
 
 
+@pytest.mark.parametrize('kind', ['gdn', 'm2'])
+@pytest.mark.parametrize('top', [1e-30, 1.0, 1e30, 3e38])
+def test_bf16_states_over_the_whole_range(kind, top):
+    """One token on bf16 states from tiny to the format's largest values, every output against 64 bits (128 products and
+    their fp32 sum: 2e-5 of the largest output, as everywhere)."""
+    hv, hk, dk, dv, B = 4, 2, 128, 64, 3
+    g0 = torch.Generator().manual_seed(12)
+    lay = (SlotLayout if kind == 'gdn' else Mamba2SlotLayout)('bf16', hv, hk, dk, dv, m=8, buffer_bits=8)
+    blob = lay.alloc(B + 1, DEV)
+    V = lay.views(blob)
+    idx = torch.arange(1, B + 1, dtype=torch.int32, device=DEV)
+    S0 = (torch.rand(B, hv, dv, dk, generator=g0) * 2 - 1) * top
+    S0[torch.rand(S0.shape, generator=g0) > 1 / 16] *= 2.0 ** -6     # few enough of the largest for the results to be finite
+    lay.write(V, idx, S0.to(DEV))
+    S = V['S'][idx.long()].view(B, hv, dv, dk).double()
+    assert top < 1e38 or S.abs().max() > 2.9e38
+    q, k = (torch.randn(B, hk, dk, generator=g0).to(DEV) for _ in range(2))
+    v = torch.randn(B, hv, dv, generator=g0).to(DEV)
+    out = torch.empty(B, hv, dv, device=DEV)
+    up = lambda x: x.double().repeat_interleave(hv // hk, 1)                              # noqa: E731
+    if kind == 'gdn':
+        g, beta = (-torch.rand(B, hv, generator=g0)).to(DEV), torch.rand(B, hv, generator=g0).to(DEV)
+        lay.step(V, idx, q, k, v, out, dk ** -0.5, g=g, beta=beta)
+        qn = up(q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6)) * dk ** -0.5
+        kn = up(k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6))
+        a = g.double().exp()[..., None]
+        u = beta.double()[..., None] * (v.double() - a * torch.einsum('bhvk,bhk->bhv', S, kn))
+        want = a * torch.einsum('bhvk,bhk->bhv', S, qn) + (qn * kn).sum(-1, keepdim=True) * u
+    else:
+        A, dt = -torch.rand(hv, generator=g0).to(DEV), torch.rand(B, hv, generator=g0).to(DEV)
+        q *= 2.0 ** -10                                      # C: keeps the largest outputs inside fp32
+        lay.step(V, idx, v, dt, k, q, out, A, D=None, dt_bias=None, dt_softplus=False)
+        a = (dt * A).double().exp()[..., None]
+        want = a * torch.einsum('bhvk,bhk->bhv', S, up(q)) + (up(q) * up(k)).sum(-1, keepdim=True) * (dt[..., None] * v).double()
+    err = ((out.double() - want).abs().max() / want.abs().max()).item()
+    assert err < 2e-5, err                                   # (false for a NaN)
+
+
 INT4V_128 = dict(kind='gdn', fmt=(4, 'v', 32), B=1, hv=4, hk=2, dk=128, dv=128, m=8, bb=8, T=17, seed=73)
 
 
