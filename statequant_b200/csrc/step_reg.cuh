@@ -225,9 +225,10 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     const FxScale fq = fx_scale<TOP>(mq), fk = fx_scale<TOP>(mk);
 #pragma unroll
     for (int j = 0; j < CW; j++) {
+      if (KIND == K_M2) d += kr[j] * qr[j];                // C . B as it is
       qr[j] = (qr[j] * fq.m1) * fq.m2;
       kr[j] = (kr[j] * fk.m1) * fk.m2;
-      d += kr[j] * qr[j];
+      if (KIND != K_M2) d += kr[j] * qr[j];                // (the vectors' norms still missing, so not to overflow or vanish)
     }
     // bf16: the state pass's fragments: lane l's columns 4 l .. 4 l + 3 are step l / 8 * 2 + l % 2, thread (l % 8) / 2
     if constexpr (!QUANT) {
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   // first power, so that no step between lies beyond the sum and the result: states near the largest float)
   const float iq1 = KIND == K_M2 ? misc[4] : misc[4] * misc[8], iq2 = misc[5];
   const float ik1 = KIND == K_M2 ? misc[6] : misc[6] * misc[9], ik2 = misc[7];
-  const float kq = (((misc[0] * iq1) * iq2) * ik1) * ik2;
+  const float kq = KIND == K_M2 ? misc[0] : (((misc[0] * iq1) * iq2) * ik1) * ik2;
   const int n0 = __float_as_int(misc[1]);                  // live buffer entries of this slot
   const bool full = n0 == M - 1;                           // this token fills the buffer: fold after the read-out
   if (warp == 3 && first) {
