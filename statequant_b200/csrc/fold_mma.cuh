@@ -43,6 +43,10 @@ __device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], uint32_t saddr) {
 __device__ __forceinline__ void stsm_x2(uint32_t saddr, uint32_t r0, uint32_t r1) {
   asm volatile("stmatrix.sync.aligned.m8n8.x2.shared.b16 [%0], {%1, %2};" ::"r"(saddr), "r"(r0), "r"(r1) : "memory");
 }
+__device__ __forceinline__ void st_v8(float* p, float a, float b, float c, float d, float e, float f, float g, float h) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h) : "memory");
+}
 __device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
@@ -328,7 +332,9 @@ __device__ __forceinline__ float fold_round(const float (&acc)[NH][4][4], int la
 // key scale (both are in the key fragments, three bf16 planes: build_key_frags_kda), and a product L Kd is taken as
 // p1 r1 + p1 r2 + p2 r1 + p1 r3 + p2 r2 + p3 r1 (the three terms left out are below 2^-24 of it).
 // READ: nothing is rounded or written back; the accumulators, i.e. the state advanced across the buffer, go to
-// out [stage rows][DK] fp32 instead (a thread's four adjacent columns of a row as one 16-byte store).
+// out [stage rows][DK] fp32 instead.  A thread of a quad has four adjacent columns of a row (8-bit: the quad stores 64 bytes at a
+// time) or eight (4-bit): a whole 32-byte sector, stored as one where out allows.  As two 16-byte stores each writes half a
+// sector, and the read-out is bound by the sectors it writes: 256 rows of 32 heads 149 us, 116 us as one.
 //
 // Bound by instruction issue (with its share of the step around it).  Two halves (64 columns, 32 values of a thread) are
 // taken at once: independent chains for the scheduler, and the 2 or 4 fresh scales of a quad (rows x groups) are
@@ -346,6 +352,7 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
   const int hh = (g * R) / DV;                         // head of this thread's rows within the stage
   const float* tb = tab + hh * TABW;
   const float2 al2 = make_float2(tb[16], tb[16]);
+  [[maybe_unused]] const bool sectors = (reinterpret_cast<uintptr_t>(out) & 31) == 0;     // out on a 32-byte boundary: st_v8
   auto block = [&](int bb) {
     const int b = 2 * w + bb;
     const int row0 = g * R + 2 * b;                    // stage rows row0, row0 + 1
@@ -386,9 +393,13 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
 #pragma unroll
           for (int r = 0; r < 2; r++) {
             float* p0 = o0 + r * DK + fold_col<BITS>(h0 + h, 0, t);
-            *reinterpret_cast<float4*>(p0) = make_float4(acc[h][0][2 * r], acc[h][0][2 * r + 1], acc[h][1][2 * r], acc[h][1][2 * r + 1]);
-            *reinterpret_cast<float4*>(p0 + (BITS == 8 ? 16 : 4)) =
-                make_float4(acc[h][2][2 * r], acc[h][2][2 * r + 1], acc[h][3][2 * r], acc[h][3][2 * r + 1]);
+            const auto& v = acc[h];
+            if (BITS == 4 && sectors) {
+              st_v8(p0, v[0][2 * r], v[0][2 * r + 1], v[1][2 * r], v[1][2 * r + 1], v[2][2 * r], v[2][2 * r + 1], v[3][2 * r], v[3][2 * r + 1]);
+            } else {
+              *reinterpret_cast<float4*>(p0) = make_float4(v[0][2 * r], v[0][2 * r + 1], v[1][2 * r], v[1][2 * r + 1]);
+              *reinterpret_cast<float4*>(p0 + (BITS == 8 ? 16 : 4)) = make_float4(v[2][2 * r], v[2][2 * r + 1], v[3][2 * r], v[3][2 * r + 1]);
+            }
           }
         }
         return;
@@ -406,23 +417,12 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
         stsm_x2(addr, o[0][0], o[0][1]);
       }
     };
-    if constexpr (READ && BITS == 4) {
-#pragma unroll
-      for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
-    } else {
 #pragma unroll 1
-      for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
-    }
+    for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
     if constexpr (NHALF % 2 == 1) chunk(IntC<1>(), NHALF - 1);
   };
-  // (the 4-bit read-out unrolled: 82 rows of 16 heads 30.4 -> 29.4 us; 8-bit, 256 rows: 121.9 as a loop, 123.5 unrolled)
-  if constexpr (READ && BITS == 4) {
-#pragma unroll
-    for (int bb = 0; bb < 2; bb++) block(bb);
-  } else {
 #pragma unroll 1
-    for (int bb = 0; bb < 2; bb++) block(bb);
-  }
+  for (int bb = 0; bb < 2; bb++) block(bb);
 }
 
 // The same fold for 4-bit codes scaled along v in groups of 32 rows (one scale per column and group).  Warp w owns

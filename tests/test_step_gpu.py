@@ -426,6 +426,29 @@ def test_device_read_write_match_torch(kind, fmt):
     assert int(V['NPTR'][idx.long(), 0].max()) == 5         # reading leaves the slots alone
 
 
+@pytest.mark.parametrize('kind,fmt', [('gdn', (4, 'k', 64)), ('gdn', (8, 'k', 32)), ('gdn', (4, 'v', 32)), ('m2', (4, 'k', 64))])
+def test_slot_read_into_any_16_byte_boundary(kind, fmt):
+    """``sqb_slot_read`` takes an output on any 16-byte boundary (its stores are 16 bytes wide, or 32 where the output allows):
+    the same values at every offset, and nothing outside them written."""
+    import ctypes as C
+    from statequant_b200 import _cabi
+    P, g0 = 3, torch.Generator().manual_seed(6)
+    lay = SlotLayout(sq.Quantizer(*fmt), 4, 2, 128, 128, m=8) if kind == 'gdn' else Mamba2SlotLayout(sq.Quantizer(*fmt), 4, 2, 128, 128, m=8)
+    blob = lay.alloc(P + 1, DEV)
+    V = lay.views(blob)
+    idx = torch.arange(1, P + 1, dtype=torch.int32, device=DEV)
+    lay.write(V, idx, (torch.randn(P, 4, 128, 128, generator=g0) * 0.5).to(DEV))
+    want = lay.read(V, idx).flatten()
+    for off in (0, 4, 8, 12):                                # floats
+        raw = torch.full((want.numel() + 32,), 7., device=DEV)
+        out = raw[8 + off:8 + off + want.numel()]
+        assert out.data_ptr() % 32 == 4 * off % 32
+        _cabi.check(_cabi.lib().sqb_slot_read(C.byref(lay._struct(V)), lay.kind, idx.data_ptr(), P, out.data_ptr(),
+                                              _cabi.current_stream(idx.device)), 'sqb_slot_read')
+        assert torch.equal(out, want)
+        assert (raw[:8 + off] == 7.).all() and (raw[8 + off + want.numel():] == 7.).all()
+
+
 def _full_batch(lay, steps, make, run_dev, run_oracle, sample_n=4, hv=None, dv=None):
     """BASELINE-size batch through the device twice (determinism), padding rows, and a sample of rows against the
     oracle from their pre-step bytes, across one fold period."""
