@@ -19,10 +19,10 @@ constexpr float FP16_TINY = 5.960464477539063e-08f;   // 2^-24
 constexpr float FP16_MIN_NORMAL = 6.103515625e-05f;   // 2^-14
 constexpr float MAGIC = 12582912.0f;                  // 1.5 * 2^23: adding it rounds to an integer (half-even)
 
-// Programmatic dependent launch: every kernel of this library is launched so that its CTAs may become resident while the
-// kernel in front of it on the stream still runs (launch_pdl in launchers.h).  dependency_wait() stands in front of a
-// kernel's first access to global memory and returns once that kernel has finished and its writes are visible;
-// dependency_release(), after it, lets the next kernel's CTAs in as soon as all of this one's are resident.
+// Programmatic dependent launch: a kernel launched with launch_pdl (launchers.h) may have its CTAs resident while the kernel in
+// front of it on the stream still runs.  dependency_wait() stands in front of every kernel's first access to global memory
+// and returns once that kernel has finished and its writes are visible; dependency_release(), after it, lets the next
+// kernel's CTAs in as soon as all of this one's are resident.  The fold launch decides per size (fold_launch.cu).
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -1,6 +1,6 @@
 // The fold as its own launch, right after the step kernel of the same call.
 //
-// On a slot's m-th token the staged step kernel only appends: it leaves the head's counter at m
+// On a slot's m-th token the step kernel in front of it only appends: it leaves the head's counter at m
 // (a value that never survives the call), the running log decay in GCUR and the buffer complete.  This kernel then
 // rewrites the stored state of exactly those heads,
 //     S = exp(gcur) S_0 + sum_i (exp(gcur - G_i) u_i) k_i^T      (KDA: the decay ratio sits on the key, per channel)
@@ -55,22 +55,28 @@ __host__ __device__ inline SmemF smemf_plan(bool vdec, int bits, int axk, int gr
   return s;
 }
 
+// What an instance carries: FOLD_ANY the fp32 fold of any shape, which also reads (out given); FOLD_TENS and READ_TENS the
+// tensor-pipe code (fold_mma.cuh) for Gated DeltaNet / Mamba2 heads of 128 x 128 with a buffer of 8.  One kernel for all three
+// spills 64 bytes and slows each of them: 4-bit d_v 192, 64 rows of 32 heads, slots mixed 45.3 us per layer-step against 44.3;
+// int8 k/32, 256 rows 64.8 against 63.4.
+enum { FOLD_ANY = 0, FOLD_TENS = 1, READ_TENS = 2 };
+
 struct FoldArgs {
   uint8_t *S, *SC, *KB, *KBS, *UB, *UBS, *GB, *GCUR, *NPTR;
   long long sS, sSC, sKB, sKBS, sUB, sUBS, sGB, sGC, sN;
   const int* idx;
   int group, qbuf, M, HV, HK, DV, rows;
   int* status;
-  int tens;                  // the fold on the tensor pipe (fold_mma.cuh): Gated DeltaNet / Mamba2 heads of 128 x 128, buffer of 8
+  int release;               // let the next kernel's CTAs in before this one has finished (fold_launch.cu)
   float* out;                // read mode: fp32 [rows, HV, d_v, d_k], the state advanced across its pending buffer
 };
 
-template <bool VDEC, int BITS, bool AXK, int LPR>
+template <bool VDEC, int BITS, bool AXK, int LPR, int MODE>
 __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ FoldArgs A, const __grid_constant__ SmemF P) {
   dependency_wait();
-  dependency_release();
+  if (A.release) dependency_release();
   constexpr int DK = LPR * 16;
-  constexpr bool TENS_OK = !VDEC && AXK && LPR == 8;       // instantiations that carry the tensor-pipe fold
+  constexpr bool TENS = MODE != FOLD_ANY;
   extern __shared__ __align__(128) uint8_t smraw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int DV = A.DV, M = A.M, HV = A.HV, G = A.group;
@@ -109,7 +115,7 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
     const long long seq = slot_of(pair);
     uint8_t* st = smraw + P.stage0 + s * P.stage_bytes;
     mbar_expect_tx(&bars[s], stage_tx);
-    if (TENS_OK && A.tens) {                   // eight pieces of 16 rows, 16 bytes apart (mma_pass.cuh)
+    if (TENS) {                  // eight pieces of 16 rows, 16 bytes apart (mma_pass.cuh)
       constexpr int PB = 16 * (DK * BITS / 8);
       for (int l = 0; l < 8; l++) bulk_g2s(st + l * (PB + 16), A.S + seq * A.sS + (long long)h * P.codes_b + l * PB, PB, &bars[s]);
     } else {
@@ -136,7 +142,7 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
       long long seq = b;
       bool live = true;
       if (A.idx != nullptr) { seq = A.idx[b]; live = seq > 0; }
-      if (live) due = A.out != nullptr || reinterpret_cast<const int*>(A.NPTR + seq * A.sN)[h] == M;
+      if (live) due = (TENS ? MODE == READ_TENS : A.out != nullptr) || reinterpret_cast<const int*>(A.NPTR + seq * A.sN)[h] == M;
     }
     const unsigned bal = __ballot_sync(0xffffffffu, due);
     int wbase = 0;
@@ -170,7 +176,7 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
       // small per-head scalars straight from global memory while the copies land
       float gnew = 0.f;
       if (!VDEC) gnew = *GCh;
-      const bool reading = A.out != nullptr;
+      const bool reading = TENS ? MODE == READ_TENS : A.out != nullptr;
       const int nlive = reading ? (reinterpret_cast<const int*>(A.NPTR + seq * A.sN)[h] & (M - 1)) : M;   // buffer entries in use
       const bool landed = mbar_wait(&bars[s], (phases >> s) & 1);
       phases ^= 1u << s;
@@ -179,60 +185,58 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
         failed = true;
         break;
       }
-      if constexpr (TENS_OK) {
-        if (A.tens) {
-          // ---- the fold on the tensor pipe, from the stage as padded pieces, written back by bulk copies ----
-          constexpr int UPG = BITS == 8 ? 1 : 2, ROWB = DK * BITS / 8, PITCH = 16 * ROWB + 16;
-          float* tab = R;                              // dec_i, value scales, alpha (R and L are free in this mode)
-          uint32_t* KBf = reinterpret_cast<uint32_t*>(R + 32);
-          float* udq = L;
-          if (reading) {
-            // the state advanced across the nlive <= 7 pending slots; dead slots (any bytes) count as zero
-            if (tid < 8) {
-              const bool lv = tid < nlive;
-              tab[tid] = lv ? expf(gnew - GBh[tid]) : 0.f;
-              tab[8 + tid] = lv ? h2f(UBSh[tid]) : 0.f;
-              ksf[tid] = lv ? h2f(KBSh[tid]) : 0.f;
-              if (tid == 0) tab[16] = expf(gnew);
-            }
-            udq[tid] = 0.f;
-            build_key_frags<BITS>(KBf, reinterpret_cast<const int8_t*>(kbt), reinterpret_cast<const int8_t*>(kbt) + 7 * DK, tid);
-            __syncthreads();
-            fold_stage_mma<BITS, UPG, 128, false, true>(smem_u32(st), reinterpret_cast<unsigned short*>(st + P.o_sc),
-                                                        reinterpret_cast<const int8_t*>(ubt), udq, tab, ksf, KBf, warp, lane, nullptr,
-                                                        A.out + (long long)pair * DV * DK);
-            __syncthreads();                           // the stage, the tables and the fragments are free
-            if (tid == 0 && e + 2 < cnt) {
-              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-              issue(s, list[e + 2]);
-            }
-            continue;
-          }
+      if constexpr (TENS) {
+        // ---- the fold on the tensor pipe, from the stage as padded pieces, written back by bulk copies ----
+        constexpr int UPG = BITS == 8 ? 1 : 2, ROWB = DK * BITS / 8, PITCH = 16 * ROWB + 16;
+        float* tab = R;                              // dec_i, value scales, alpha (R and L are free in this mode)
+        uint32_t* KBf = reinterpret_cast<uint32_t*>(R + 32);
+        float* udq = L;
+        if constexpr (MODE == READ_TENS) {
+          // the state advanced across the nlive <= 7 pending slots; dead slots (any bytes) count as zero
           if (tid < 8) {
-            tab[tid] = tid == 7 ? 1.0f : expf(gnew - GBh[tid]);
-            tab[8 + tid] = h2f(UBSh[tid]);
-            ksf[tid] = h2f(KBSh[tid]);
+            const bool lv = tid < nlive;
+            tab[tid] = lv ? expf(gnew - GBh[tid]) : 0.f;
+            tab[8 + tid] = lv ? h2f(UBSh[tid]) : 0.f;
+            ksf[tid] = lv ? h2f(KBSh[tid]) : 0.f;
             if (tid == 0) tab[16] = expf(gnew);
           }
-          udq[tid] = static_cast<float>(reinterpret_cast<const int8_t*>(ubt)[7 * DV + tid]) * h2f(UBSh[7]);   // d_v = 128 = NT
+          udq[tid] = 0.f;
           build_key_frags<BITS>(KBf, reinterpret_cast<const int8_t*>(kbt), reinterpret_cast<const int8_t*>(kbt) + 7 * DK, tid);
           __syncthreads();
-          fold_stage_mma<BITS, UPG, 128, false>(smem_u32(st), reinterpret_cast<unsigned short*>(st + P.o_sc),
-                                                reinterpret_cast<const int8_t*>(ubt), udq, tab, ksf, KBf, warp, lane);
-          if (tid == 0) { *GCh = 0.f; reinterpret_cast<int*>(A.NPTR + seq * A.sN)[h] = 0; }
-          __syncthreads();
-          if (warp == 0) {
+          fold_stage_mma<BITS, UPG, 128, false, true>(smem_u32(st), reinterpret_cast<unsigned short*>(st + P.o_sc),
+                                                      reinterpret_cast<const int8_t*>(ubt), udq, tab, ksf, KBf, warp, lane, nullptr,
+                                                      A.out + (long long)pair * DV * DK);
+          __syncthreads();                           // the stage, the tables and the fragments are free
+          if (tid == 0 && e + 2 < cnt) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            uint8_t* Sg = A.S + seq * A.sS + (long long)h * P.codes_b;
-            if (lane < 8) bulk_s2g(Sg + lane * 16 * ROWB, st + lane * PITCH, 16 * ROWB);
-            else if (lane == 8) bulk_s2g(A.SC + seq * A.sSC + (long long)h * scn * 2, st + P.o_sc, scn * 2);
-            bulk_commit();
-            bulk_wait_read();                          // the stage may be refilled, and the CTA may leave
-            __syncwarp();
-            if (lane == 0 && e + 2 < cnt) issue(s, list[e + 2]);
+            issue(s, list[e + 2]);
           }
           continue;
         }
+        if (tid < 8) {
+          tab[tid] = tid == 7 ? 1.0f : expf(gnew - GBh[tid]);
+          tab[8 + tid] = h2f(UBSh[tid]);
+          ksf[tid] = h2f(KBSh[tid]);
+          if (tid == 0) tab[16] = expf(gnew);
+        }
+        udq[tid] = static_cast<float>(reinterpret_cast<const int8_t*>(ubt)[7 * DV + tid]) * h2f(UBSh[7]);   // d_v = 128 = NT
+        build_key_frags<BITS>(KBf, reinterpret_cast<const int8_t*>(kbt), reinterpret_cast<const int8_t*>(kbt) + 7 * DK, tid);
+        __syncthreads();
+        fold_stage_mma<BITS, UPG, 128, false>(smem_u32(st), reinterpret_cast<unsigned short*>(st + P.o_sc),
+                                              reinterpret_cast<const int8_t*>(ubt), udq, tab, ksf, KBf, warp, lane);
+        if (tid == 0) { *GCh = 0.f; reinterpret_cast<int*>(A.NPTR + seq * A.sN)[h] = 0; }
+        __syncthreads();
+        if (warp == 0) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          uint8_t* Sg = A.S + seq * A.sS + (long long)h * P.codes_b;
+          if (lane < 8) bulk_s2g(Sg + lane * 16 * ROWB, st + lane * PITCH, 16 * ROWB);
+          else if (lane == 8) bulk_s2g(A.SC + seq * A.sSC + (long long)h * scn * 2, st + P.o_sc, scn * 2);
+          bulk_commit();
+          bulk_wait_read();                          // the stage may be refilled, and the CTA may leave
+          __syncwarp();
+          if (lane == 0 && e + 2 < cnt) issue(s, list[e + 2]);
+        }
+        continue;
       }
       if (tid < M) {
         if (!VDEC) dec[tid] = tid >= nlive ? 0.f : (!reading && tid == M - 1 ? 1.0f : expf(gnew - GBh[tid]));

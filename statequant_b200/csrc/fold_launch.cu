@@ -7,9 +7,9 @@
 namespace sqb {
 namespace {
 
-template <bool VDEC, int BITS, bool AXK, int LPR>
-int launch_fold_one(const StepArgs& a, cudaStream_t stream, float* out) {
-  auto kern = fold_kernel<VDEC, BITS, AXK, LPR>;
+template <bool VDEC, int BITS, bool AXK, int LPR, int MODE>
+int launch_fold_mode(const StepArgs& a, cudaStream_t stream, float* out) {
+  auto kern = fold_kernel<VDEC, BITS, AXK, LPR, MODE>;
   const SmemF plan = smemf_plan(VDEC, BITS, AXK, a.group, a.DK, a.DV, a.M, a.qbuf);
   if (plan.total > 220 * 1024) return 1;
   static SmemLimit limit;                   // per instantiation
@@ -29,21 +29,35 @@ int launch_fold_one(const StepArgs& a, cudaStream_t stream, float* out) {
   f.idx = a.idx; f.group = a.group; f.qbuf = a.qbuf; f.M = a.M; f.HV = a.HV; f.HK = a.HK; f.DV = a.DV; f.rows = a.rows;
   f.status = a.status;
   f.out = out;
-  f.tens = !VDEC && AXK && LPR == 8 && a.DV == 128 && a.M == 8 && a.qbuf &&
-           ((BITS == 8 && a.group == 32) || (BITS == 4 && a.group == 64));
   const long long pairs = static_cast<long long>(a.rows) * a.HV;
   int per_sm = (220 * 1024) / (plan.total + 1024);
   if (per_sm > 4) per_sm = 4;
   if (per_sm < 1) per_sm = 1;
-  long long grid = static_cast<long long>(nsm) * per_sm;
-  if (grid > pairs) grid = pairs;
-  // The read-out is launched without the early entry of launch_pdl: a persistent grid whose CTAs move in as the kernel in front
-  // of it leaves ends up bunched on the SMs that were free first (its first CTAs, with a pair more, on the same ones): 82
-  // rows of 16 heads 33.3 us a read against 30.4, 64 rows of 32 heads (4-bit, v/32) 58.4 against 52.2.
-  const dim3 g3(static_cast<unsigned>(grid));
-  const cudaError_t e = out != nullptr ? launch_plain(kern, g3, NT, plan.total, stream, f, plan) : launch_pdl(kern, g3, NT, plan.total, stream, f, plan);
+  const long long wave = static_cast<long long>(nsm) * per_sm;
+  const dim3 grid(static_cast<unsigned>(pairs < wave ? pairs : wave));
+  // Which of this kernel and its neighbours on the stream may overlap (us per layer-step of the two-launch paths; launches as in
+  // stream order / this kernel let in early (launch_pdl) / the next kernel let in early (release) / both).  CTAs let in early
+  // take the SMs that are free first.  That pays while no CTA has more than two pairs: int8 k/32, 4 rows of 32 heads 8.5 / 7.7 /
+  // 8.3 / 8.0, 16 rows 12.1 / 11.8 / 12.3 / 12.8; int4 k/64, 24 rows 9.8 / 9.1 / 10.3 / 10.5; d_v 192, 16 rows 24.4 / 24.2 / 29.9
+  // / 32.8.  A longer grid ends up bunched, its first CTAs, with a pair more, on the same SMs: int8 k/32, 256 rows with every
+  // slot due 51.5 / 58.8 / 50.9 / 58.0; d_k 64, 64 rows 15.4 / 14.8 / 15.6 / 15.9.  Decays per channel (KDA: the step kernel behind it
+  // has the longest prologue) gain from the release at any size, 4 rows 10.9 / 11.4 / 10.1 / 10.1, 64 rows 37.2 / 43.1 / 36.7 / 39.7.
+  // The read-out, with a slot write behind it: 64 rows of 32 heads 73 / 74 / 79 / 80 us a pair of calls.
+  const bool early = out == nullptr && !VDEC && pairs <= 2 * wave;
+  f.release = out == nullptr && VDEC;
+  const cudaError_t e = early ? launch_pdl(kern, grid, NT, plan.total, stream, f, plan) : launch_plain(kern, grid, NT, plan.total, stream, f, plan);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
+}
+
+template <bool VDEC, int BITS, bool AXK, int LPR>
+int launch_fold_one(const StepArgs& a, cudaStream_t stream, float* out) {
+  if constexpr (!VDEC && AXK && LPR == 8) {
+    if (a.DV == 128 && a.M == 8 && a.qbuf && a.group == (BITS == 8 ? 32 : 64))
+      return out != nullptr ? launch_fold_mode<VDEC, BITS, AXK, LPR, READ_TENS>(a, stream, out)
+                            : launch_fold_mode<VDEC, BITS, AXK, LPR, FOLD_TENS>(a, stream, out);
+  }
+  return launch_fold_mode<VDEC, BITS, AXK, LPR, FOLD_ANY>(a, stream, out);
 }
 
 template <bool VDEC>

@@ -556,6 +556,72 @@ def test_two_devices_in_one_process():
     assert res[0][0].any()
 
 
+@pytest.mark.parametrize('kind,fmt,dv,path', [('gdn', (8, 'k', 32), 128, 3), ('gdn', (4, 'k', 64), 192, 0), ('kda', (4, 'k', 64), 128, 3),
+                                             ('gdn', (8, 'k', 32), 128, 0)])
+@pytest.mark.parametrize('rows', [5, 38])
+def test_overlapping_launches_equal_separate_ones(kind, fmt, dv, path, rows):
+    """Layers stepped back to back in a CUDA graph, where a kernel's CTAs may enter while the kernel before it drains, give the
+    bytes of the same calls with a device-wide wait after each.  32 heads, slots on different tokens: fold launches of less
+    than a wave of CTAs (5 rows) and of more than two (38); copies and a fork in between; two fold periods."""
+    from statequant_b200 import _cabi
+    L, T, H, D = 3, 9, 32, 128
+    g0 = torch.Generator().manual_seed(31)
+    n = lambda *s: torch.randn(*s, generator=g0)                                          # noqa: E731
+    lay = (KDASlotLayout(sq.Quantizer(*fmt), H, D, dv, m=8) if kind == 'kda' else
+           SlotLayout(sq.Quantizer(*fmt), H, H // 2, D, dv, m=8))
+    hk = H if kind == 'kda' else H // 2
+    blob = torch.zeros(L, rows + 1, lay.nbytes, dtype=torch.uint8, device=DEV)
+    idx = (torch.randperm(rows, generator=g0) + 1).to(torch.int32).to(DEV)
+    for layer in range(L):
+        lay.write(lay.views(blob[layer]), idx, (n(1, H, dv, D).expand(rows, -1, -1, -1) * 0.5).to(DEV))
+    g = -torch.rand(rows, H, D, generator=g0) * 0.1 if kind == 'kda' else -torch.rand(rows, H, generator=g0) * 0.1
+    x = [t.to(DEV) for t in (n(rows, hk, D).bfloat16(), n(rows, hk, D).bfloat16(), n(rows, H, dv).bfloat16(), g, torch.rand(rows, H, generator=g0))]
+    out = torch.zeros(L, T, rows, H, dv, dtype=torch.bfloat16, device=DEV)
+    side = torch.cuda.Stream()
+
+    def step(V, i, o):
+        if kind == 'kda':
+            lay.step(V, i, *x, o, D ** -0.5)
+        else:
+            lay.step(V, i, x[0], x[1], x[2], o, D ** -0.5, g=x[3], beta=x[4])
+
+    def burst(out, wait):
+        for t in range(T):
+            for layer in range(L):
+                step(lay.views(blob[layer]), idx, out[layer, t])
+                wait()
+                if layer == 0:                                # a copy node in front of the next step
+                    spare.copy_(out[0, t])
+                    wait()
+            if t == 3:                                        # and a branch that joins in front of one
+                side.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(side):
+                    spare2.copy_(out[1, t])
+                torch.cuda.current_stream().wait_stream(side)
+
+    _cabi.set_option('kernel_path', path)
+    try:
+        spare, spare2 = torch.empty_like(out[0, 0]), torch.empty_like(out[0, 0])
+        for t in range(8):                                    # slots on tokens of their own
+            step(lay.views(blob[0]), torch.where(torch.arange(rows, device=DEV) % 8 > t, idx, 0), out[0, 0])
+        blob[1:] = blob[0]
+        keep = blob.clone()
+        burst(out, torch.cuda.synchronize)
+        want_out, want = out.clone(), blob.clone()
+        torch.cuda.synchronize()
+        G = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(G):
+            burst(out, lambda: None)
+        for _ in range(3):
+            blob.copy_(keep)
+            out.zero_()
+            G.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(out, want_out) and torch.equal(blob, want)
+    finally:
+        _cabi.set_option('kernel_path', 0)
+
+
 LONG_TAIL = [
     dict(kind='gdn', fmt=(8, 'k', 32), B=2, hv=4, hk=2, dk=128, dv=192, m=8, bb=8, seed=41),
     dict(kind='gdn', fmt=(4, 'k', 64), B=2, hv=4, hk=2, dk=128, dv=192, m=8, bb=8, seed=42),
