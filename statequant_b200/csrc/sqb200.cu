@@ -29,6 +29,8 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
+constexpr long long SMS = 148;             // of a B200: the launch rules below are drawn for it
+
 bool pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 int ilog2(int x) { int l = 0; while ((1 << l) < x) l++; return l; }
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -121,7 +123,12 @@ int launch_one(const sqb::StepArgs& a, cudaStream_t stream) {
   }
   const long long ctas = static_cast<long long>(a.rows) * a.HV;
   if (ctas > 2147483647LL) return fail(SQB_EINVAL, "rows * hv = %lld exceeds the grid limit", ctas);
-  const cudaError_t e = sqb::launch_pdl(kern, dim3(static_cast<unsigned>(ctas)), sqb::NT, smem, stream, a);
+  // States scaled along v fold in one long CTA per head: where SMs hold more than one, those let in early crowd on the SMs that are
+  // free first (4-bit, 96 x 192, 30 heads, us per token in stream order / let in early: 4 rows 37.8 / 37.2, 8 rows 63.2 / 65.0 and, all
+  // slots due, 22.7 / 24.9, 32 rows 103.6 / 107.4).  The other formats gain at any size (fp32 128 x 128, 32 heads: 32 rows 71.8 / 71.1).
+  const dim3 grid(static_cast<unsigned>(ctas));
+  const cudaError_t e = AXK || ctas <= SMS ? sqb::launch_pdl(kern, grid, sqb::NT, smem, stream, a)
+                                           : sqb::launch_plain(kern, grid, sqb::NT, smem, stream, a);
   if (e != cudaSuccess) return fail(SQB_ECUDA, "kernel launch: %s", cudaGetErrorString(e));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
@@ -189,7 +196,7 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
   // per-CTA work counts.  us per layer and token, tensor-core kernel -> this one, int8 k/32, 32 heads of 128 x 128, slots
   // folding together / each on a token of its own: 1 row 4.9 -> 3.2 / 4.9 -> 3.2, 8 rows 5.2 -> 3.9 / 10.0 -> 6.0, 16 rows (512
   // CTAs) 5.9 -> 5.6 / 11.6 -> 7.8, 24 rows 8.2 -> 8.7 / 16.2 -> 10.8, 256 rows 44.9 -> 60.2 / 57.9 -> 63.3.
-  constexpr long long ONE_WAVE = 4 * 148;
+  constexpr long long ONE_WAVE = 4 * SMS;
   if (path != 1 && sqb::reg_shape_ok(a0, bits, axk, KIND)) {
     const bool few = static_cast<long long>(a0.rows) * (a0.HV / (a0.DV == 64 ? 2 : 1)) <= ONE_WAVE;
     if (path == 5 || (path == 0 && few) || !sqb::mma_shape_ok(a0, bits, axk, kda, KIND))
