@@ -237,6 +237,8 @@ const char *sqb_last_error(void);
 int sqb_abi_version(void);
 /* number of kernel launches issued by this library in this process (all threads) */
 int64_t sqb_launch_count(void);
+/* decode-step calls (GDN, Mamba2, KDA) that ran on kernel path 1 .. 5 (see sqb_set_option), in this process; -1: no such path */
+int64_t sqb_path_count(int path);
 /* tuning / test switches.
    "kernel_path" selects the kernel of the decode steps: 0 the best one for the shape (default); 1 the generic kernel
    (direct loads, folds inside its own launch; any supported shape); 2 the staged SIMT kernel (one CTA per batch row

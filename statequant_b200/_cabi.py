@@ -94,7 +94,8 @@ def lib():
         L = C.CDLL(LIB_PATH)
         L.sqb_last_error.restype = C.c_char_p
         L.sqb_abi_version.restype = C.c_int
-        L.sqb_launch_count.restype = C.c_int64
+        L.sqb_launch_count.restype = L.sqb_path_count.restype = C.c_int64
+        L.sqb_path_count.argtypes = [C.c_int]
         for name in ('sqb_gdn_step', 'sqb_mamba2_step', 'sqb_kda_step', 'sqb_gga_step'):
             f = getattr(L, name)
             f.restype = C.c_int
@@ -129,6 +130,11 @@ def current_stream(device):
 
 def launch_count():
     return int(lib().sqb_launch_count())
+
+
+def path_counts():
+    """Decode-step calls by the kernel path they ran on (1 .. 5, as ``kernel_path`` numbers them)."""
+    return {p: int(lib().sqb_path_count(p)) for p in range(1, 6)}
 
 
 def set_option(name, value):

@@ -20,6 +20,7 @@ namespace {
 
 thread_local char g_err[512] = "";
 std::atomic<long long> g_launches{0};
+std::atomic<long long> g_paths[6];         // step calls by the kernel path they took
 
 int fail(int code, const char* fmt, ...) {
   va_list ap;
@@ -185,6 +186,12 @@ bool fold_fits(const sqb::StepArgs& a, int bits, bool axk, bool kda) {
   return sqb::smemf_plan(kda, bits, axk, a.group, a.DK, a.DV, a.M, a.qbuf).total <= 220 * 1024;
 }
 
+// a step call has been launched on kernel path p (rc 0) or refused
+int took(int p, int rc) {
+  if (rc == 0) g_paths[p].fetch_add(1, std::memory_order_relaxed);
+  return rc;
+}
+
 template <int KIND>
 int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
   const sqb::StepArgs& a = a0;
@@ -200,7 +207,7 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
   if (path != 1 && sqb::reg_shape_ok(a0, bits, axk, KIND)) {
     const bool few = static_cast<long long>(a0.rows) * (a0.HV / (a0.DV == 64 ? 2 : 1)) <= ONE_WAVE;
     if (path == 5 || (path == 0 && few) || !sqb::mma_shape_ok(a0, bits, axk, kda, KIND))
-      return sub_rc(sqb::launch_reg(KIND, a0, bits, stream));
+      return took(5, sub_rc(sqb::launch_reg(KIND, a0, bits, stream)));
   }
   // Every check that could refuse a launch is made before the first one: a positive "shape not taken" code after a
   // step kernel has appended would leave the slot between two states.
@@ -209,17 +216,17 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
     a.axv = axk ? 0 : 1;
     sqb::SmemM plan;
     int nst;
-    if ((path == 4 || path == 0) && sqb::mma_fold_inside(a, bits, KIND)) {
+    if ((path == 0 || path >= 4) && sqb::mma_fold_inside(a, bits, KIND)) {
       // tensor-core kernel with the fold inside: one launch, the stored state read once per token
       if (sqb::mma_plan<KIND>(a, bits, 3, plan, nst)) {
         const int rc = launch_mma_kind<KIND>(a, bits, 3, stream);
-        return rc <= 0 ? rc : fail(SQB_ECUDA, "tensor-core step kernel refused a checked shape");
+        return rc <= 0 ? took(4, rc) : fail(SQB_ECUDA, "tensor-core step kernel refused a checked shape");
       }
     } else if (sqb::mma_plan<KIND>(a, bits, 0, plan, nst) && fold_fits(a, bits, axk, kda)) {
       const int rc = launch_mma_kind<KIND>(a, bits, 0, stream);
       if (rc != 0) return rc < 0 ? rc : fail(SQB_ECUDA, "tensor-core step kernel refused a checked shape");
       const int rf = sub_rc(sqb::launch_fold(KIND, a, bits, axk, stream));
-      return rf <= 0 ? rf : fail(SQB_ECUDA, "fold kernel refused a checked shape");
+      return rf <= 0 ? took(3, rf) : fail(SQB_ECUDA, "fold kernel refused a checked shape");
     }
   }
   if (path != 1 && tma_ok(a, bits, axk, kda) && fold_fits(a, bits, axk, kda)) {
@@ -229,14 +236,14 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
     if (rc < 0) return rc;
     if (rc == 0) {
       const int rf = sub_rc(sqb::launch_fold(KIND, a, bits, axk, stream));
-      return rf <= 0 ? rf : fail(SQB_ECUDA, "fold kernel refused a checked shape");
+      return rf <= 0 ? took(2, rf) : fail(SQB_ECUDA, "fold kernel refused a checked shape");
     }
   }
   switch (bits) {
-    case 4: return axk ? launch_one<KIND, 4, true>(a, stream) : launch_one<KIND, 4, false>(a, stream);
-    case 8: return axk ? launch_one<KIND, 8, true>(a, stream) : launch_one<KIND, 8, false>(a, stream);
-    case 16: return launch_one<KIND, 16, true>(a, stream);
-    case 32: return launch_one<KIND, 32, true>(a, stream);
+    case 4: return took(1, axk ? launch_one<KIND, 4, true>(a, stream) : launch_one<KIND, 4, false>(a, stream));
+    case 8: return took(1, axk ? launch_one<KIND, 8, true>(a, stream) : launch_one<KIND, 8, false>(a, stream));
+    case 16: return took(1, launch_one<KIND, 16, true>(a, stream));
+    case 32: return took(1, launch_one<KIND, 32, true>(a, stream));
   }
   return fail(SQB_ENOTBUILT, "no kernel for %d-bit states", bits);
 }
@@ -253,6 +260,7 @@ extern "C" {
 const char* sqb_last_error(void) { return g_err; }
 int sqb_abi_version(void) { return 1; }
 int64_t sqb_launch_count(void) { return g_launches.load(); }
+int64_t sqb_path_count(int path) { return path >= 1 && path <= 5 ? g_paths[path].load() : -1; }
 
 int sqb_set_option(const char* name, int value) {
   if (name && !strcmp(name, "force_generic_kernel")) { g_force_generic = value; return 0; }

@@ -750,6 +750,55 @@ def test_bf16_states_over_the_whole_range(kind, top):
     assert err < 2e-5, err                                   # (false for a NaN)
 
 
+def _one_step(kind, fmt, dk, dv, hv, hk, m, bb, rows):
+    lay = (SlotLayout(fmt if isinstance(fmt, str) else sq.Quantizer(*fmt), hv, hk, dk, dv, m=m, buffer_bits=bb) if kind == 'gdn' else
+           Mamba2SlotLayout(fmt if isinstance(fmt, str) else sq.Quantizer(*fmt), hv, hk, dk, dv, m=m, buffer_bits=bb) if kind == 'm2' else
+           KDASlotLayout(sq.Quantizer(*fmt), hv, dk, dv, m=m, buffer_bits=bb))
+    blob = lay.alloc(2, DEV)                                 # one slot; the other rows are padding
+    idx = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    idx[0] = 1
+    z = lambda *s: torch.zeros(*s, device=DEV)                                            # noqa: E731
+    V, out = lay.views(blob), z(rows, hv, dv)
+    if kind == 'gdn':
+        lay.step(V, idx, z(rows, hk, dk), z(rows, hk, dk), z(rows, hv, dv), out, 1.0, g=z(rows, hv), beta=z(rows, hv))
+    elif kind == 'm2':
+        lay.step(V, idx, z(rows, hv, dv), z(rows, hv), z(rows, hk, dk), z(rows, hk, dk), out, z(hv))
+    else:
+        lay.step(V, idx, z(rows, hv, dk), z(rows, hv, dk), z(rows, hv, dv), z(rows, hv, dk), z(rows, hv), out)
+
+
+# kind, format, d_k, d_v, heads, m, buffer bits, rows, kernel_path -> the path that runs
+ROUTES = [
+    ('gdn', (8, 'k', 32), 128, 128, (32, 16), 8, 8, 18, 0, 5), ('gdn', (8, 'k', 32), 128, 128, (32, 16), 8, 8, 19, 0, 4),   # 592 CTAs
+    ('gdn', (4, 'k', 64), 128, 128, (8, 4), 8, 8, 74, 0, 5), ('gdn', (4, 'k', 64), 128, 128, (8, 4), 8, 8, 75, 0, 4),
+    ('m2', (8, 'k', 32), 128, 64, (128, 8), 8, 8, 9, 0, 5), ('m2', (8, 'k', 32), 128, 64, (128, 8), 8, 8, 10, 0, 4),
+    ('gdn', (8, 'k', 32), 128, 128, (32, 16), 8, 8, 4, 3, 3), ('gdn', (8, 'k', 32), 128, 128, (32, 16), 8, 8, 40, 5, 5),
+    ('gdn', 'bf16', 128, 128, (32, 16), 8, 8, 40, 0, 5), ('gdn', 'bf16', 128, 64, (3, 3), 8, 8, 1, 5, 1),
+    ('gdn', 'bf16', 128, 128, (4, 2), 8, 16, 1, 5, 1), ('gdn', 'bf16', 128, 128, (4, 2), 4, 8, 1, 0, 1),
+    ('gdn', (4, 'k', 64), 96, 192, (30, 30), 8, 8, 40, 0, 5), ('gdn', (4, 'v', 32), 96, 192, (30, 30), 8, 8, 1, 0, 1),
+    ('gdn', 'fp32', 128, 128, (4, 2), 8, 8, 1, 5, 1),
+    # path 5 on shapes the register-tile kernel does not take: the tensor-core kernel with its fold inside, as path 4
+    ('gdn', (4, 'v', 32), 128, 128, (4, 2), 8, 8, 1, 5, 4), ('gdn', (8, 'k', 64), 128, 128, (4, 2), 8, 8, 1, 5, 4),
+    ('kda', (4, 'k', 64), 128, 128, (4, 4), 8, 8, 1, 5, 4), ('gdn', (8, 'k', 32), 128, 128, (4, 2), 16, 8, 1, 5, 3),
+    ('gdn', (8, 'k', 32), 64, 64, (4, 2), 8, 8, 1, 5, 2), ('gdn', (8, 'k', 32), 128, 128, (4, 2), 8, 8, 1, 1, 1),
+]
+
+
+@pytest.mark.parametrize('kind,fmt,dk,dv,heads,m,bb,rows,path,want', ROUTES)
+def test_kernel_path_taken(kind, fmt, dk, dv, heads, m, bb, rows, path, want):
+    """Which kernel a call runs on, by shape, grid and ``kernel_path``; a path that does not take a shape falls through to the next
+    lower one (the header's contract)."""
+    from statequant_b200 import _cabi
+    _cabi.set_option('kernel_path', path)
+    try:
+        before = _cabi.path_counts()
+        _one_step(kind, fmt, dk, dv, *heads, m, bb, rows)
+        torch.cuda.synchronize()
+        assert {p: n - before[p] for p, n in _cabi.path_counts().items()} == {p: int(p == want) for p in range(1, 6)}
+    finally:
+        _cabi.set_option('kernel_path', 0)
+
+
 INT4V_128 = dict(kind='gdn', fmt=(4, 'v', 32), B=1, hv=4, hk=2, dk=128, dv=128, m=8, bb=8, T=17, seed=73)
 
 
