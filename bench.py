@@ -566,8 +566,9 @@ def main():
     ap.add_argument('--workload', default='gdn', choices=list(WORKLOADS),
                     help='gdn = the benchmark; mamba2 / kda / gga time the other kernel families on their shapes')
     ap.add_argument('--mma-hpc', type=int, default=0, help='tensor-core kernels: value heads per CTA (0: a whole key head)')
-    ap.add_argument('--kernel-path', type=int, default=0, choices=[0, 1, 2, 3, 4],
-                    help='0 best kernel for the shape; 1 generic; 2 staged + fold launch (profiling / comparison)')
+    ap.add_argument('--kernel-path', type=int, default=0, choices=[0, 1, 2, 3, 4, 5],
+                    help='0 best kernel for the shape; 1 generic; 2 staged + fold launch; 3 tensor-core step + fold launch; 4 with the '
+                         'fold inside; 5 register tile (profiling / comparison)')
     ap.add_argument('--conv-only', action='store_true',
                     help='time only the causal conv update in front of the step (--layers caches in rotation) and print its figures')
     args = ap.parse_args()

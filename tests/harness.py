@@ -123,6 +123,7 @@ def replay_vs_golden(name, c, oracle=None, device='cpu', act_dtype=torch.float32
         a = {k: v.to(device) for k, v in step_args(c, inp, t, act_dtype).items()}
         run_step(c, lay, V, idx, a, out, inp, oracle=oracle)
         want = _tt(G['o'][t], device).view(B, hv, dv)
+        assert not out.isnan().any(), t                           # (max() below passes over a NaN)
         st['worst'] = max(st['worst'], ((out - want).abs().max() / want.abs().max()).item())
         kc, uc = _tt(G['Kc'][t], device), _tt(G['Uc'][t], device)
         if c['bb'] == 16:

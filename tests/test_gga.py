@@ -1,5 +1,6 @@
 """GGA / STEP mixed-bit state with the pure-write window: the oracle against golden vectors of the reference's torch
 code (CPU), and the CUDA kernels against the oracle on the same slot bytes and against the golden record (GPU)."""
+import numpy as np
 import pytest
 import torch
 
@@ -20,6 +21,46 @@ def _setup(c, device='cpu'):
     blob = torch.randint(0, 256, (c['B'] + 2, pk.nbytes + 64), dtype=torch.uint8, generator=g)[:, :pk.nbytes]
     blob[:, :16] = 0                                             # counters of unused slots: sane
     return pk, bits, w, blob.to(device) if device != 'cpu' else blob
+
+
+def test_refit_by_rows_weights_keeps_the_precision():
+    """The register-tile step refits a column factor as c = sum (w r)^2 z y / sum (w r)^2 z^2 with y = x / r rounded to fp32, where
+    the reference has sum w^2 (r z) x / sum w^2 (r z)^2: the same sums in fp32 (16 rows in order, then 8 partials) against 64
+    bits.  The error of the rewritten form is no larger (rms; within 5 %, a sample's spread)."""
+    r, f = np.random.RandomState(0), np.float32
+    fma = lambda a, b, c: (a.astype(np.float64) * b + c).astype(f)                        # noqa: E731
+    rows = lambda k: np.arange(8) * 16 + k                                                # noqa: E731
+
+    def total(parts):
+        t = parts[0]
+        for p in parts[1:]:
+            t = t + p
+        return t
+
+    sq_err, n = np.zeros(2), 0
+    for bits in (4, 6):
+        qmax = (1 << (bits - 1)) - 1
+        for _ in range(20):
+            x = (r.standard_normal((128, 128)) * np.exp(r.standard_normal((128, 1)))).astype(f)
+            w = (r.rand(128, 1) + 0.5).astype(f)
+            rf = np.sqrt(np.abs(x).mean(1, keepdims=True) / w).astype(np.float16).astype(f)
+            y = x / rf
+            z = np.clip(np.rint(y / (np.abs(y).max(0) / f(qmax)).astype(np.float16).astype(f)), -qmax, qmax).astype(f)
+            W, V = w.astype(np.float64) ** 2, rf.astype(np.float64) * z
+            want = (W * V * x).sum(0) / (W * V * V).sum(0)
+            num, den, num2, den2 = (np.zeros((8, 128), f) for _ in range(4))
+            v, ww, wr = rf * z, w * w, (w * rf) * (w * rf)
+            for k in range(16):
+                i = rows(k)
+                num, den = num + (ww[i] * v[i]) * x[i], den + ww[i] * (v[i] * v[i])
+                num2, den2 = fma(wr[i], z[i] * y[i], num2), fma(wr[i], z[i] * z[i], den2)
+            for j, c in enumerate((total(num) / total(den), total(num2) / total(den2))):
+                assert c.dtype == f
+                sq_err[j] += (((c - want) / want) ** 2).sum()
+            n += 128
+    rms = np.sqrt(sq_err / n)
+    print(f'\nrefit, relative error against 64 bits (rms): {rms[0]:.2e} as the reference writes it, {rms[1]:.2e} by row weights')
+    assert rms[1] <= 1.05 * rms[0] and rms[1] < 1.2e-7
 
 
 def test_fit_matches_reference():
