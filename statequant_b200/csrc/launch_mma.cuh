@@ -90,7 +90,11 @@ int launch_mma_one_io(const StepArgs& a, cudaStream_t stream) {
   while ((1 << b.m_log2) < a.M) b.m_log2++;
   if (a.HV / b.hpc > 65535) return 1;
   const dim3 grid(static_cast<unsigned>(a.rows), static_cast<unsigned>(a.HV / b.hpc));
-  const cudaError_t e = launch_pdl(kern, grid, NT, plan.total, stream, b, plan, nst);
+  static Residency residency;               // per instantiation
+  // (a step kernel with a fold launch behind it always enters early: its neighbour is another kernel, fold_launch.cu)
+  const bool early = MODE != 3 || enters_early(ctas, residency.ctas(kern, NT, plan.total), KIND == K_KDA);
+  const cudaError_t e = early ? launch_pdl(kern, grid, NT, plan.total, stream, b, plan, nst)
+                              : launch_plain(kern, grid, NT, plan.total, stream, b, plan, nst);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
 }

@@ -49,6 +49,32 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, size_t smem, 
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
+// CTAs of a kernel that the current device holds at once, asked once per device and shared-memory size.
+struct Residency {
+  std::atomic<long long> known[64];              // smem << 32 | CTAs
+  template <class K>
+  long long ctas(K kern, int threads, int smem) {
+    int dev = 0, nsm = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const long long k = known[dev & 63].load(std::memory_order_relaxed);
+    if (dev < 64 && k != 0 && (k >> 32) == smem) return k & 0xFFFFFFFFll;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess)
+      return 0;
+    const long long all = static_cast<long long>(nsm) * n;
+    if (dev < 64) known[dev].store(static_cast<long long>(smem) << 32 | all, std::memory_order_relaxed);
+    return all;
+  }
+};
+// Whether a step kernel of `grid` CTAs enters early, where the GPU holds `all`: the CTAs of two launches find room side by side up to
+// half of it, and from about 0.8 of it on they fill every SM however they come in.  Between the two they crowd on the SMs that are
+// free first.  us per layer-step in stream order / early, all slots due together: tensor-core kernel, int4 k/64 (740 at once) 320 CTAs
+// 7.0 / 6.7, 384 7.1 / 8.2, 576 8.1 / 8.5, 640 8.9 / 8.6, 1024 14.1 / 13.6; int8 v/32 (592) 288 CTAs 7.9 / 7.5, 304 8.5 / 9.1, 384 8.7 /
+// 9.2, 512 9.9 / 9.4; Mamba2 int8 320 7.3 / 6.8, 384 7.4 / 8.5, 640 9.9 / 9.5; register tile, int8 k/32 (592) 288 CTAs 4.3 / 4.0, 320 4.9 /
+// 5.5, 416 5.0 / 5.6, 512 5.9 / 5.6; bf16 1024 13.3 / 12.8.  KDA (one head per CTA: the folding ones end the launch) crowds up to a whole
+// wave where slots are due one in eight: 608 CTAs 12.1 / 12.9, 736 12.8 / 13.4 (all due 7.8 / 7.6, 8.3 / 7.8), 1024 17.6 / 17.4.
+inline bool enters_early(long long grid, long long all, bool kda) { return 2 * grid <= all || (kda ? grid > all : 5 * grid > 4 * all); }
+
 // Shapes the register-tile step takes: d_k 128 and d_v 64 or 128 with bf16 states or (Gated DeltaNet, Mamba2) 8-bit codes in
 // key groups of 32 or 4-bit codes in key groups of 64; Gated DeltaNet states of d_k 96 and d_v 64, 128 or 192 with those codes;
 // decays per head, int8 buffer of 8, q / k per key head, a CTA's rows of one key head.

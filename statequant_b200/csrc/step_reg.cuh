@@ -532,8 +532,10 @@ int launch_reg_one(const StepArgs& a, cudaStream_t stream) {
   const dim3 grid(static_cast<unsigned>(a.rows), static_cast<unsigned>(a.HV / HPS));
   // bf16 activations and output take the kernel with those element types compiled in
   const bool bio = a.dt_qk == DT_BF16 && a.dt_v == DT_BF16 && a.dt_out == DT_BF16;
-  const cudaError_t e = bio ? launch_pdl(step_reg_kernel<KIND, BITS, DK, DV, HPS, true>, grid, HPS * DV, 0, stream, b)
-                            : launch_pdl(step_reg_kernel<KIND, BITS, DK, DV, HPS, false>, grid, HPS * DV, 0, stream, b);
+  auto kern = bio ? step_reg_kernel<KIND, BITS, DK, DV, HPS, true> : step_reg_kernel<KIND, BITS, DK, DV, HPS, false>;
+  static Residency residency[2];
+  const bool early = enters_early(static_cast<long long>(grid.x) * grid.y, residency[bio].ctas(kern, HPS * DV, 0), false);
+  const cudaError_t e = early ? launch_pdl(kern, grid, HPS * DV, 0, stream, b) : launch_plain(kern, grid, HPS * DV, 0, stream, b);
   return e == cudaSuccess ? 0 : -(1000 + static_cast<int>(e));
 }
 

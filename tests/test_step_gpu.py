@@ -572,11 +572,11 @@ def test_two_devices_in_one_process():
 
 @pytest.mark.parametrize('kind,fmt,dv,path', [('gdn', (8, 'k', 32), 128, 3), ('gdn', (4, 'k', 64), 192, 0), ('kda', (4, 'k', 64), 128, 3),
                                              ('gdn', (8, 'k', 32), 128, 0), ('gdn', (4, 'v', 32), 128, 1)])
-@pytest.mark.parametrize('rows', [4, 38])
+@pytest.mark.parametrize('rows', [4, 24, 38])
 def test_overlapping_launches_equal_separate_ones(kind, fmt, dv, path, rows):
     """Layers stepped back to back in a CUDA graph, where a kernel's CTAs may enter while the kernel before it drains, give the
-    bytes of the same calls with a device-wide wait after each.  32 heads, slots on different tokens: grids of less than a
-    wave of CTAs (4 rows) and of more than two (38); copies and a fork in between; two fold periods."""
+    bytes of the same calls with a device-wide wait after each.  32 heads, slots on different tokens: grids of less than half a
+    wave of CTAs (4 rows), of about half of one (24) and of more than two (38); copies and a fork in between; two fold periods."""
     from statequant_b200 import _cabi
     L, T, H, D = 3, 9, 32, 128
     g0 = torch.Generator().manual_seed(31)
