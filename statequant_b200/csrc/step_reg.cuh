@@ -2,8 +2,7 @@
 // along k (groups of 64 / 32, the last one of 96 columns short); decays per head (Gated DeltaNet, Mamba2), int8 buffer of 8,
 // q / k per key head.
 //
-// One CTA per (batch row, ROWS state rows), a thread per row: one head of d_v 128 or 192, two heads of d_v 64 (of one key
-// head).  Warp w owns rows 32 w .. 32 w + 31 = two blocks of 16; lane (g, t) = (lane / 4, lane % 4) loads rows g and g + 8 of
+// One CTA per batch row and head, a thread per state row: a head of d_v 128 or 192, or two heads of d_v 64 (of one key head).  Warp w owns rows 32 w .. 32 w + 31 = two blocks of 16; lane (g, t) = (lane / 4, lane % 4) loads rows g and g + 8 of
 // a block, columns 32 j + 8 t .. + 7 of every unit j of 32 columns: one load each (16 bytes of bf16, 8 of int8, 4 of int4),
 // all requested before anything waits.  A loaded word is a register of a matrix instruction's A fragment as it stands (the
 // order of the columns along the contraction is free as long as B follows it) and, on the token that folds, part of a C
@@ -22,6 +21,10 @@
 // Measured per layer and token, generic kernel -> this one (the generic kernel's CTA goes through six block reductions before
 // its state pass and holds 12 warps per SM): bf16, 96 rows of 32 heads of 128 x 128, 120 -> 29.6 us (18 us at the copy rate);
 // 4-bit, 64 rows of 30 heads of 96 x 192, a slot in eight folding, 103 -> 25.2 us.  Against the tensor-core kernel: sqb200.cu.
+//
+// Not taken, and left to the kernels that had them: integer states scaled along v (a column's scale would have to go into the
+// vectors, a set of fragments per scale group), decays per key channel (fragments per buffer slot), other key groups than those
+// of the presets, and d_k 96 with bf16 states or Mamba2.
 #pragma once
 #include "launchers.h"
 #include "step_tma.cuh"
@@ -31,7 +34,8 @@ namespace sqb {
 
 // Threads per SM: bf16 holds 64 words of state per thread (128 registers); integer states of d_k 128 come here in grids of up
 // to four CTAs per SM, and need the registers more than the residency; those of d_k 96 in grids of any size (80 registers:
-// 852 us a pass against 955 us with 112).
+// 852 us a pass against 955 us with 112).  What the caps cost (ptxas): 96-wide instances spill 16 .. 56 bytes (28 .. 68 loaded), bf16
+// ones 12 .. 24 (16 .. 40), 8-bit ones of d_k 128 up to 16, 4-bit ones of d_k 128 nothing.
 constexpr int reg_min_ctas(int bits, int dk, int threads) { return (bits == 16 || dk == 128 ? 512 : 768) / threads; }
 
 // N words of a lane's slice of a unit: 4 (bf16), 2 (int8) or 1 (int4)

@@ -188,7 +188,9 @@ def fold_policy():
 
 def apply_fold_policy():
     """Select the device code path of the decode steps for this process: kernel_path 3 (step kernel that only appends +
-    the fold launch) for 'launch', 0 (the fold inside the step kernel wherever the shape allows) for 'inline'."""
+    the fold launch; shapes that step kernel does not take run on the register-tile, staged or generic kernel) for 'launch', 0 (no
+    second launch wherever the shape allows: the register-tile kernel for grids of one wave, the fold inside the step kernel
+    above that) for 'inline'."""
     from .. import _cabi
     _cabi.set_option('kernel_path', 3 if fold_policy() == 'launch' else 0)
 

@@ -15,8 +15,7 @@ from .layout import KIND_GDN, BlobLayout, set_shape
 
 
 def _gdn_inputs(idx, q, k, v, out, scale, g, beta, gate, per_key_head):
-    """Assemble ``sqb_gdn_inputs_t`` for tensors laid out [rows, heads, dim] (or [rows * heads, dim] for the
-    lockstep container, which passes explicit strides through 3-d views)."""
+    """Assemble ``sqb_gdn_inputs_t`` for tensors laid out [rows, heads, dim]."""
     assert k.dtype == q.dtype
     stride, code = _cabi.row_stride_bytes, _cabi.dtype_code
     if gate is not None:
