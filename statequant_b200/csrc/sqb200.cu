@@ -200,9 +200,12 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
   // The register-tile kernel (step_reg.cuh): shapes the tensor-core kernel does not take, and grids that fit the GPU at once
   // (its CTAs are resident four to an SM).  There the serial chain of a CTA is what counts: it spreads a row over twice as many
   // warps (a head per CTA) and reads and folds without a detour through shared memory.  In longer grids its larger share of
-  // per-CTA work counts.  us per layer and token, tensor-core kernel -> this one, int8 k/32, 32 heads of 128 x 128, slots
-  // folding together / each on a token of its own: 1 row 4.9 -> 3.2 / 4.9 -> 3.2, 8 rows 5.2 -> 3.9 / 10.0 -> 6.0, 16 rows (512
-  // CTAs) 5.9 -> 5.6 / 11.6 -> 7.8, 24 rows 8.2 -> 8.7 / 16.2 -> 10.8, 256 rows 44.9 -> 60.2 / 57.9 -> 63.3.
+  // per-CTA work counts.  us per layer and token, tensor-core kernel -> this one, slots folding together / an eighth of them on
+  // each token: int8 k/32, 32 heads of 128 x 128: 1 row 4.9 -> 3.3 / 5.0 -> 3.3, 8 rows 5.3 -> 4.1 / 12.3 -> 7.2, 18 rows (576 CTAs) 6.8
+  // -> 6.4 / 15.0 -> 9.8, 19 rows (608) 7.2 -> 8.6 / 14.2 -> 10.6, 37 rows 10.0 -> 11.5 / 21.9 -> 15.0; int4 k/64: 16 rows 6.3 -> 5.1 / 14.5 ->
+  // 8.2, 19 rows 6.7 -> 7.3 / 13.8 -> 9.3; Mamba2, 128 heads of 64 rows, int8: 8 rows (512) 7.1 -> 6.1 / 15.3 -> 9.1, 10 rows (640) 8.0 -> 8.7
+  // / 16.5 -> 10.6; int4: 6.2 -> 4.9 / 14.1 -> 8.1, 6.7 -> 7.6 / 15.0 -> 9.5.  In all four formats slots that fold together turn at one wave;
+  // where they do not is known to the device only.
   constexpr long long ONE_WAVE = 4 * SMS;
   if (path != 1 && sqb::reg_shape_ok(a0, bits, axk, KIND)) {
     const bool few = static_cast<long long>(a0.rows) * (a0.HV / (a0.DV == 64 ? 2 : 1)) <= ONE_WAVE;
