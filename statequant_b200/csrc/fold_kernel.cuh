@@ -33,17 +33,17 @@ __host__ __device__ inline SmemF smemf_plan(bool vdec, int bits, int axk, int gr
   s.kb_b = al16i(M * DK * bsz);
   s.gb_b = vdec ? M * DK * 4 : 0;
   s.gc_b = vdec ? DK * 4 : 0;
-  s.o_sc = s.codes_b + 128;                 // (room for the padded-piece layout of the tensor-pipe fold)
+  s.o_sc = s.codes_b;
   s.o_ub = s.o_sc + s.scales_b;
   s.o_kb = s.o_ub + s.ub_b;
   s.o_gb = s.o_kb + s.kb_b;
   s.o_gc = s.o_gb + s.gb_b;
-  s.stage_bytes = s.o_gc + s.gc_b;
+  s.stage_bytes = (s.o_gc + s.gc_b + 1023) & ~1023;         // (the swizzle of the tensor-pipe fold's copies repeats every 1024 bytes)
   int o = 0;
+  s.stage0 = o; o += 2 * s.stage_bytes;
   s.bars = o; o += 64;
   s.list = o; o += 128 * 4 + 64;            // pairs found in one scan round (+ counters)
   o = (o + 127) & ~127;
-  s.stage0 = o; o += 2 * s.stage_bytes;
   s.f0 = o;
   int f = 0;
   s.R = f; f += M * s.rdk;
@@ -72,12 +72,13 @@ struct FoldArgs {
 };
 
 template <bool VDEC, int BITS, bool AXK, int LPR, int MODE>
-__global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ FoldArgs A, const __grid_constant__ SmemF P) {
+__global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ FoldArgs A, const __grid_constant__ TileMap codes_map,
+                                                      const __grid_constant__ SmemF P) {
   dependency_wait();
   if (A.release) dependency_release();
   constexpr int DK = LPR * 16;
   constexpr bool TENS = MODE != FOLD_ANY;
-  extern __shared__ __align__(128) uint8_t smraw[];
+  extern __shared__ __align__(1024) uint8_t smraw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int DV = A.DV, M = A.M, HV = A.HV, G = A.group;
   const int gqa = HV / A.HK;
@@ -115,9 +116,8 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
     const long long seq = slot_of(pair);
     uint8_t* st = smraw + P.stage0 + s * P.stage_bytes;
     mbar_expect_tx(&bars[s], stage_tx);
-    if (TENS) {                  // eight pieces of 16 rows, 16 bytes apart (mma_pass.cuh)
-      constexpr int PB = 16 * (DK * BITS / 8);
-      for (int l = 0; l < 8; l++) bulk_g2s(st + l * (PB + 16), A.S + seq * A.sS + (long long)h * P.codes_b + l * PB, PB, &bars[s]);
+    if (TENS) {                  // swizzled (mma_pass.cuh)
+      tile_g2s(st, &codes_map, h * DV, static_cast<int>(seq), &bars[s]);
     } else {
       bulk_g2s(st, A.S + seq * A.sS + (long long)h * P.codes_b, P.codes_b, &bars[s]);
     }
@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
         break;
       }
       if constexpr (TENS) {
-        // ---- the fold on the tensor pipe, from the stage as padded pieces, written back by bulk copies ----
-        constexpr int UPG = BITS == 8 ? 1 : 2, ROWB = DK * BITS / 8, PITCH = 16 * ROWB + 16;
+        // ---- the fold on the tensor pipe, from the stage, written back by bulk copies ----
+        constexpr int UPG = BITS == 8 ? 1 : 2;
         float* tab = R;                              // dec_i, value scales, alpha (R and L are free in this mode)
         uint32_t* KBf = reinterpret_cast<uint32_t*>(R + 32);
         float* udq = L;
@@ -225,12 +225,11 @@ __global__ void __launch_bounds__(NT, 4) fold_kernel(const __grid_constant__ Fol
         fold_stage_mma<BITS, UPG, 128, false>(smem_u32(st), reinterpret_cast<unsigned short*>(st + P.o_sc),
                                               reinterpret_cast<const int8_t*>(ubt), udq, tab, ksf, KBf, warp, lane);
         if (tid == 0) { *GCh = 0.f; reinterpret_cast<int*>(A.NPTR + seq * A.sN)[h] = 0; }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (warp == 0) {
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          uint8_t* Sg = A.S + seq * A.sS + (long long)h * P.codes_b;
-          if (lane < 8) bulk_s2g(Sg + lane * 16 * ROWB, st + lane * PITCH, 16 * ROWB);
-          else if (lane == 8) bulk_s2g(A.SC + seq * A.sSC + (long long)h * scn * 2, st + P.o_sc, scn * 2);
+          if (lane == 0) tile_s2g(&codes_map, h * DV, static_cast<int>(seq), st);
+          else if (lane == 1) bulk_s2g(A.SC + seq * A.sSC + (long long)h * scn * 2, st + P.o_sc, scn * 2);
           bulk_commit();
           bulk_wait_read();                          // the stage may be refilled, and the CTA may leave
           __syncwarp();

@@ -2,6 +2,7 @@
 #include <atomic>
 #include "launchers.h"
 #include "fold_kernel.cuh"
+#include "tile_map.h"
 #include "slot_io.cuh"
 
 namespace sqb {
@@ -43,9 +44,13 @@ int launch_fold_mode(const StepArgs& a, cudaStream_t stream, float* out) {
   // slot due 51.5 / 58.8 / 50.9 / 58.0; d_k 64, 64 rows 15.4 / 14.8 / 15.6 / 15.9.  Decays per channel (KDA: the step kernel behind it
   // has the longest prologue) gain from the release at any size, 4 rows 10.9 / 11.4 / 10.1 / 10.1, 64 rows 37.2 / 43.1 / 36.7 / 39.7.
   // The read-out, with a slot write behind it: 64 rows of 32 heads 73 / 74 / 79 / 80 us a pair of calls.
+  TileMap map{};
+  if (MODE != FOLD_ANY) {
+    if (const int e = tile_map(map, a, BITS)) return -1000 - e;
+  }
   const bool early = out == nullptr && !VDEC && pairs <= 2 * wave;
   f.release = out == nullptr && VDEC;
-  const cudaError_t e = early ? launch_pdl(kern, grid, NT, plan.total, stream, f, plan) : launch_plain(kern, grid, NT, plan.total, stream, f, plan);
+  const cudaError_t e = early ? launch_pdl(kern, grid, NT, plan.total, stream, f, map, plan) : launch_plain(kern, grid, NT, plan.total, stream, f, map, plan);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
 }
@@ -53,7 +58,7 @@ int launch_fold_mode(const StepArgs& a, cudaStream_t stream, float* out) {
 template <bool VDEC, int BITS, bool AXK, int LPR>
 int launch_fold_one(const StepArgs& a, cudaStream_t stream, float* out) {
   if constexpr (!VDEC && AXK && LPR == 8) {
-    if (a.DV == 128 && a.M == 8 && a.qbuf && a.group == (BITS == 8 ? 32 : 64))
+    if (a.DV == 128 && a.M == 8 && a.qbuf && a.group == (BITS == 8 ? 32 : 64) && tile_map_ok(a))
       return out != nullptr ? launch_fold_mode<VDEC, BITS, AXK, LPR, READ_TENS>(a, stream, out)
                             : launch_fold_mode<VDEC, BITS, AXK, LPR, FOLD_TENS>(a, stream, out);
   }

@@ -50,6 +50,16 @@ __device__ __forceinline__ void st_v8(float* p, float a, float b, float c, float
 __device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
+// One copy of a box of a tensor map (64- or 128-byte rows of a slot's codes, swizzled in shared memory: mma_pass.cuh); x = 0 always.
+struct alignas(64) TileMap { unsigned char bytes[128]; };      // a CUtensorMap, encoded by the host (tile_map.h)
+__device__ __forceinline__ void tile_g2s(void* dst, const TileMap* map, int row, int slot, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(smem_u32(dst)), "l"(map), "r"(0), "r"(row), "r"(slot), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tile_s2g(const TileMap* map, int row, int slot, const void* src) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];"
+               ::"l"(map), "r"(0), "r"(row), "r"(slot), "r"(smem_u32(src)) : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // the bulk stores of this thread have read their shared-memory source (which may then be reused or released)
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -324,8 +334,9 @@ __device__ __forceinline__ float fold_round(const float (&acc)[NH][4][4], int la
   return s_own;
 }
 
-// Folds the 32 rows of warp w (row blocks 2w and 2w + 1) of a stage of eight pieces of R rows.
-//   st_addr / scs: the stage's codes (padded pieces) and scales [row][NG] in shared memory, both rewritten in place
+// Folds the 32 rows of warp w (two row blocks) of a stage.
+//   st_addr / scs: the stage's codes and scales [row][NG] in shared memory, both rewritten in place.  The codes lie as the tensor-map
+//   copy swizzles them (mma_pass.cuh: block bb = rows 32 w + 16 bb .., a thread's rows g and g + 8 of it)
 //   ubt: the stage's buffered values [heads][8][DV] int8 (slots 0..6); udq: this token's rounded values [heads][DV]
 //   tab: per head of the stage 8 floats dec_i (dec_7 unused), 8 floats value scales, then alpha; ksf: key scales [8]
 // VDEC (KDA): decays per key channel: the start value is (code scale) ae[k], ae = exp(gnew); L carries no decay and no
@@ -341,37 +352,37 @@ __device__ __forceinline__ float fold_round(const float (&acc)[NH][4][4], int la
 // reduced by a transposing butterfly, computed by ONE lane each and exchanged.  Rounding is a branch-free exact division
 // (div_round2).  Token that folds, 256 rows of 32 heads, 8-bit: 123 us (141 us one span at a time with a verified reciprocal);
 // 4-bit, 4096 rows, a slot in eight folding: 767 us (941).
-template <int BITS, int UPG, int DV, bool VDEC = false, bool READ = false, int DK = 128, int R = 16>
+template <int BITS, int UPG, int DV, bool VDEC = false, bool READ = false>
 __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short* scs, const int8_t* ubt, const float* udq,
                                                const float* tab, const float* ksf, const uint32_t* KBf, int w, int lane,
                                                const float* ae = nullptr, float* out = nullptr) {
-  constexpr int NHALF = DK / 32, NG = (NHALF + UPG - 1) / UPG, ROWB = DK * BITS / 8, PITCH = R * ROWB + 16, TABW = 20;
+  constexpr int DK = 128, NHALF = DK / 32, NG = NHALF / UPG, ROWB = DK * BITS / 8, TABW = 20;
+  constexpr int DR = 8;                                // rows between a thread's two rows of a block
   static_assert(UPG == 1 || UPG == 2, "a scale group is one or two halves");
   const int g = lane >> 2, t = lane & 3;
-  const uint32_t lrow = st_addr + (lane & 7) * PITCH + ((lane >> 3) & 1) * ROWB + (lane >> 4) * 16;
-  const int hh = (g * R) / DV;                         // head of this thread's rows within the stage
+  const uint32_t lrow = tile_lrow<BITS>(st_addr, w, lane, 0);
+  const int hh = (32 * w) / DV;                        // head of the warp's rows within the stage
   const float* tb = tab + hh * TABW;
   const float2 al2 = make_float2(tb[16], tb[16]);
   [[maybe_unused]] const bool sectors = (reinterpret_cast<uintptr_t>(out) & 31) == 0;     // out on a 32-byte boundary: st_v8
   auto block = [&](int bb) {
-    const int b = 2 * w + bb;
-    const int row0 = g * R + 2 * b;                    // stage rows row0, row0 + 1
+    const int row0 = 32 * w + 16 * bb + g;             // stage rows row0, row0 + DR
     uint32_t A1[2], A2[2], A3[2];
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      const int rv = row0 % DV + r;
+      const int rv = row0 % DV + DR * r;
       fold_left<DV, VDEC>(ubt + hh * 8 * DV + rv, udq[hh * DV + rv], tb, ksf, t, A1[r], A2[r], A3[r]);
     }
     unsigned short* srow = scs + row0 * NG;
     // NH halves from half h0 on
     auto chunk = [&](auto nh, int h0) {
       constexpr int NH = decltype(nh)::value, NS = UPG == 1 ? NH : 1;      // halves; scale groups among them
-      const uint32_t addr = lrow + 2 * b * ROWB + (BITS == 8 ? 32 : 16) * h0;
+      const uint32_t addr = (lrow + bb * 16 * ROWB) ^ ((BITS == 8 ? 32 : 16) * h0);         // chunks of half h0 on
       const int g0 = h0 / UPG;
       uint32_t m[NH][4];                               // 8-bit: (row, row + 1) x two 16-byte pieces; 4-bit: (row, row + 1)
       if constexpr (BITS == 8) {
 #pragma unroll
-        for (int h = 0; h < NH; h++) ldsm_x4(m[h], addr + 32 * h);
+        for (int h = 0; h < NH; h++) ldsm_x4(m[h], addr ^ (32 * h));
       } else if constexpr (NH == 2) {
         uint32_t x[4];
         ldsm_x4(x, addr);
@@ -383,7 +394,7 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
       }
       float sc[2][NS];
 #pragma unroll
-      for (int s = 0; s < NS; s++) { sc[0][s] = h2f(srow[g0 + s]); sc[1][s] = h2f(srow[NG + g0 + s]); }
+      for (int s = 0; s < NS; s++) { sc[0][s] = h2f(srow[g0 + s]); sc[1][s] = h2f(srow[DR * NG + g0 + s]); }
       float acc[NH][4][4];
       fold_acc<BITS, UPG, NH, VDEC>(m, sc, A1, A2, A3, KBf, h0, lane, al2, ae, acc);
       if constexpr (READ) {
@@ -392,7 +403,7 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
         for (int h = 0; h < NH; h++) {
 #pragma unroll
           for (int r = 0; r < 2; r++) {
-            float* p0 = o0 + r * DK + fold_col<BITS>(h0 + h, 0, t);
+            float* p0 = o0 + r * DR * DK + fold_col<BITS>(h0 + h, 0, t);
             const auto& v = acc[h];
             if (BITS == 4 && sectors) {
               st_v8(p0, v[0][2 * r], v[0][2 * r + 1], v[1][2 * r], v[1][2 * r + 1], v[2][2 * r], v[2][2 * r + 1], v[3][2 * r], v[3][2 * r + 1]);
@@ -406,10 +417,10 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
       }
       uint32_t o[NH][4];
       const float s_own = fold_round<BITS, UPG, NH>(acc, lane, o);
-      if (NS == 2 || t < 2) srow[(t & 1) * NG + g0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);   // (the old scales are in registers by now)
+      if (NS == 2 || t < 2) srow[(t & 1) * DR * NG + g0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);   // (the old scales are in registers by now)
       if constexpr (BITS == 8) {
 #pragma unroll
-        for (int h = 0; h < NH; h++) stsm_x4(addr + 32 * h, o[h]);
+        for (int h = 0; h < NH; h++) stsm_x4(addr ^ (32 * h), o[h]);
       } else if constexpr (NH == 2) {
         const uint32_t x[4] = {o[0][0], o[0][1], o[1][0], o[1][1]};
         stsm_x4(addr, x);
@@ -426,7 +437,7 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
 }
 
 // The same fold for 4-bit codes scaled along v in groups of 32 rows (one scale per column and group).  Warp w owns
-// group w of the stage (the rows of tile_pass_v, mma_pass.cuh), so a column's absolute maximum over the group is a
+// group w of the stage (the warp's 32 rows), so a column's absolute maximum over the group is a
 // reduction inside the warp.  The row is walked in four chunks of 32 columns (16 bytes: one ldmatrix.x2 per 16-row
 // block); a thread holds 8 columns of 4 rows per chunk.  The reduction is a transposing butterfly over the eight lanes of
 // one t, after which lane (i, t) computes the fresh scale of ONE column (the i-th of its eight) and the lanes exchange them.
@@ -434,10 +445,10 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
 template <int DV>
 __device__ __forceinline__ void fold_stage_mma_v4(uint32_t st_addr, unsigned short* scs, const int8_t* ubt, const float* udq,
                                                   const float* tab, const float* ksf, const uint32_t* KBf, int w, int lane) {
-  constexpr int ROWB = 64, PITCH = 16 * ROWB + 16, TABW = 20;
+  constexpr int ROWB = 64, TABW = 20;
   constexpr float QMAX = 7.0f, MB = MAGIC + 8.0f;
   const int i = lane >> 2, t = lane & 3;
-  const uint32_t lrow = st_addr + (2 * w + (lane & 1)) * PITCH + (((lane & 7) >> 1) + 4 * ((lane >> 3) & 1)) * ROWB;
+  const uint32_t lrow = tile_addr<4>(st_addr, 32 * w + (lane & 15), 0);
   const int hh = (32 * w) / DV;                        // the warp's 32 rows lie in one head
   const float* tb = tab + hh * TABW;
   const float2 al2 = make_float2(tb[16], tb[16]);
@@ -447,7 +458,7 @@ __device__ __forceinline__ void fold_stage_mma_v4(uint32_t st_addr, unsigned sho
   for (int bb = 0; bb < 2; bb++) {
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      const int rv0 = (32 * w + 16 * (i & 1) + (i >> 1) + 4 * r + 8 * bb) % DV;
+      const int rv0 = (32 * w + 16 * bb + i + 8 * r) % DV;
       fold_left<DV, false>(ubt + hh * 8 * DV + rv0, udq[hh * DV + rv0], tb, ksf, t, A1[bb][r], A2[bb][r], A3[bb][r]);
     }
   }
@@ -455,8 +466,8 @@ __device__ __forceinline__ void fold_stage_mma_v4(uint32_t st_addr, unsigned sho
 #pragma unroll 1
   for (int c4 = 0; c4 < 4; c4++) {
     uint32_t wd[2][2];                                 // [block][fragment row i / i + 8]: 8 nibbles = this thread's 8 columns
-    ldsm_x2(wd[0], lrow + 16 * c4);
-    ldsm_x2(wd[1], lrow + 8 * ROWB + 16 * c4);
+    ldsm_x2(wd[0], lrow ^ (16 * c4));
+    ldsm_x2(wd[1], (lrow ^ (16 * c4)) + 16 * ROWB);
     unsigned short* scol = scs + w * 128 + 32 * c4 + 8 * t;                  // the thread's 8 column scales
     const uint4 sw = *reinterpret_cast<const uint4*>(scol);
     const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&sw.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&sw.y));
@@ -550,12 +561,12 @@ __device__ __forceinline__ void fold_stage_mma_v4(uint32_t st_addr, unsigned sho
       o[bb][1] = __byte_perm(two(by(tv[0][2], tv[0][3]), by(tv[1][2], tv[1][3])), two(by(tv[2][2], tv[2][3]), by(tv[3][2], tv[3][3])), 0x5410);
     }
     __syncwarp();                                      // every lane has read the chunk's codes
-    stsm_x2(lrow + 16 * c4, o[0][0], o[0][1]);
-    stsm_x2(lrow + 8 * ROWB + 16 * c4, o[1][0], o[1][1]);
+    stsm_x2(lrow ^ (16 * c4), o[0][0], o[0][1]);
+    stsm_x2((lrow ^ (16 * c4)) + 16 * ROWB, o[1][0], o[1][1]);
   }
 }
 
-// The same for 8-bit codes scaled along v (pieces of four rows, see tile_row_v<8>): a chunk is 32 columns = 32 bytes of
+// The same for 8-bit codes scaled along v: a chunk is 32 columns = 32 bytes of
 // a row, one ldmatrix.x4 per 16-row block; a thread holds columns 4t .. 4t + 3 and 16 + 4t .. 16 + 4t + 3 of the chunk
 // (N-block q: half q >> 1, byte pair q & 1) of four rows.
 template <int DV>
@@ -564,6 +575,7 @@ __device__ __forceinline__ void fold_stage_mma_v8(uint32_t st_addr, unsigned sho
   constexpr int TABW = 20;
   constexpr float QMAX = 127.0f, MB = MAGIC;
   const int i = lane >> 2, t = lane & 3;
+  const uint32_t lrow = tile_lrow<8>(st_addr, w, lane, 0);
   const int hh = (32 * w) / DV;
   const float* tb = tab + hh * TABW;
   const float2 al2 = make_float2(tb[16], tb[16]);
@@ -572,15 +584,15 @@ __device__ __forceinline__ void fold_stage_mma_v8(uint32_t st_addr, unsigned sho
   for (int bb = 0; bb < 2; bb++) {
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      const int rv0 = (32 * w + 4 * i + 2 * bb + r) % DV;
+      const int rv0 = (32 * w + 16 * bb + i + 8 * r) % DV;
       fold_left<DV, false>(ubt + hh * 8 * DV + rv0, udq[hh * DV + rv0], tb, ksf, t, A1[bb][r], A2[bb][r], A3[bb][r]);
     }
   }
 #pragma unroll 1
   for (int c4 = 0; c4 < 4; c4++) {
     uint32_t m[2][4];
-    ldsm_x4(m[0], tile_lrow_v<8>(st_addr, w, lane, 0) + 32 * c4);
-    ldsm_x4(m[1], tile_lrow_v<8>(st_addr, w, lane, 1) + 32 * c4);
+    ldsm_x4(m[0], lrow ^ (32 * c4));
+    ldsm_x4(m[1], (lrow ^ (32 * c4)) + 16 * 128);
     // the thread's 8 column scales: columns 4t .. 4t + 3 and 16 + 4t .. 16 + 4t + 3 of the chunk
     unsigned short* scol = scs + w * 128 + 32 * c4 + 4 * t;
     const uint2 swa = *reinterpret_cast<const uint2*>(scol), swb = *reinterpret_cast<const uint2*>(scol + 16);
@@ -673,7 +685,7 @@ __device__ __forceinline__ void fold_stage_mma_v8(uint32_t st_addr, unsigned sho
       o[2] = __byte_perm(two(u(tv[2][0]), u(tv[2][1])), two(u(tv[3][0]), u(tv[3][1])), 0x5410);
       o[3] = __byte_perm(two(u(tv[2][2]), u(tv[2][3])), two(u(tv[3][2]), u(tv[3][3])), 0x5410);
       __syncwarp();                                    // every lane has read the block's codes of this chunk
-      stsm_x4(tile_lrow_v<8>(st_addr, w, lane, bb) + 32 * c4, o);
+      stsm_x4((lrow ^ (32 * c4)) + bb * 16 * 128, o);
     }
   }
 }

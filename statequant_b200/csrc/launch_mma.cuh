@@ -3,6 +3,7 @@
 #pragma once
 #include "launchers.h"
 #include "step_mma.cuh"
+#include "tile_map.h"
 
 namespace sqb {
 
@@ -22,7 +23,7 @@ inline bool mma_shape_ok(const StepArgs& a, int bits, bool axk, bool kda, int ki
   if (gqa % hps) return false;
   if (a.M < 1 || a.M > 32 || (a.M & (a.M - 1))) return false;
   auto a16 = [](const void* p, long long s) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && s % 16 == 0; };
-  if (!a16(a.S, a.sS) || !a16(a.SC, a.sSC) || !a16(a.UB, a.sUB) || !a16(a.KB, a.sKB)) return false;
+  if (!tile_map_ok(a) || !a16(a.SC, a.sSC) || !a16(a.UB, a.sUB) || !a16(a.KB, a.sKB)) return false;
   if (((long long)a.M * a.DV) % 16) return false;
   if (kda && (!a16(a.GB, a.sGB) || !a16(a.GCUR, a.sGC))) return false;
   return true;
@@ -90,11 +91,13 @@ int launch_mma_one_io(const StepArgs& a, cudaStream_t stream) {
   while ((1 << b.m_log2) < a.M) b.m_log2++;
   if (a.HV / b.hpc > 65535) return 1;
   const dim3 grid(static_cast<unsigned>(a.rows), static_cast<unsigned>(a.HV / b.hpc));
+  TileMap map;
+  if (const int e = tile_map(map, a, BITS)) return -1000 - e;
   static Residency residency;               // per instantiation
   // (a step kernel with a fold launch behind it always enters early: its neighbour is another kernel, fold_launch.cu)
   const bool early = MODE != 3 || enters_early(ctas, residency.ctas(kern, NT, plan.total), KIND == K_KDA);
-  const cudaError_t e = early ? launch_pdl(kern, grid, NT, plan.total, stream, b, plan, nst)
-                              : launch_plain(kern, grid, NT, plan.total, stream, b, plan, nst);
+  const cudaError_t e = early ? launch_pdl(kern, grid, NT, plan.total, stream, b, map, plan, nst)
+                              : launch_plain(kern, grid, NT, plan.total, stream, b, map, plan, nst);
   if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   return 0;
 }

@@ -9,12 +9,12 @@
 // ever converted to floating point.  A fixed-point element is exact when it lies within 2^-6 of the vector's largest
 // one and is otherwise rounded to 2^-30 of it, so the pass is at least as accurate as an fp32 accumulation.
 //
-// Shared-memory layout of a head's codes ("pieces"): the d_v rows are cut into 8 pieces of R = d_v / 8 consecutive
-// rows, piece p starting at p * (R * ROWB + 16) bytes.  The 16 bytes of padding make the eight row addresses of an
-// ldmatrix 8x8 tile (one row out of each piece) fall on distinct banks; each piece is one bulk copy.
-// Fragment rows: block b (16 rows) = rows 2b and 2b + 1 of every piece; fragment row i < 8 is row 2b of piece i,
-// fragment row 8 + i is row 2b + 1 of piece i.  A warp takes blocks 2w and 2w + 1 (a tile of 32 rows) and ends up
-// with one finished row per lane: lane (i = lane / 4, t = lane % 4) owns row i * R + 4 w + t.
+// Shared-memory layout of a stage's codes (128 state rows): the rows as they lie in the slot, the 16-byte chunks of a row
+// permuted by the copy engine's swizzle (a tensor-map copy, one instruction a stage): 128-byte rows (8-bit codes) chunk ^= row
+// mod 8, 64-byte rows (4-bit) chunk ^= row / 2 mod 4, so that the eight row addresses of an ldmatrix 8x8 tile fall on distinct
+// banks.
+// A warp takes rows 32 w .. 32 w + 31 (two blocks of 16) and ends up with one finished row per lane: lane (i = lane / 4, t = lane
+// % 4) owns row 32 w + 8 t + i.
 //
 // Column n of B: vector n / 4 (0: q, 1: k), digit 3 - n % 4, so that a thread's two accumulator columns (2t, 2t + 1)
 // are the upper digit pair (t even) or the lower digit pair (t odd) of one vector.
@@ -118,27 +118,45 @@ __device__ __forceinline__ void acc_start(const uint32_t (&bf)[8], int (&ci)[4 /
   }
 }
 
+// Shared address of 16-byte chunk `chunk` of row `row` in a stage at `codes` (aligned to the swizzle's 1024 or 512 bytes).  The
+// chunk's bits are XORed with the row's, so chunk c's address is chunk 0's ^ 16 c.
+template <int BITS>
+__device__ __forceinline__ uint32_t tile_addr(uint32_t codes, int row, int chunk) {
+  constexpr int ROWB = 128 * BITS / 8;
+  return codes + row * ROWB + ((chunk ^ (BITS == 8 ? row & 7 : (row >> 1) & 3)) << 4);
+}
+// the row address this lane supplies to an ldmatrix.x4 of block bb of warp w's rows: matrices (rows 0 .. 7, rows 8 .. 15) x (chunk 0,
+// chunk 1)
+template <int BITS>
+__device__ __forceinline__ uint32_t tile_lrow(uint32_t codes, int w, int lane, int bb) {
+  return tile_addr<BITS>(codes, 32 * w + 16 * bb + (lane & 15), lane >> 4);
+}
+__device__ __forceinline__ int tile_row(int w, int lane) { return 32 * w + 8 * (lane & 3) + (lane >> 2); }
+
+// the NG fp16 scales of a row
+template <int NG>
+__device__ __forceinline__ void row_scales(const unsigned short* sc, float (&s)[NG]) {
+  if constexpr (NG == 4) {
+    const uint2 w = *reinterpret_cast<const uint2*>(sc);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+    s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
+  } else if constexpr (NG == 2) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(sc));
+    s[0] = a.x; s[1] = a.y;
+  } else {
+    s[0] = __half2float(__ushort_as_half(*sc));
+  }
+}
+
 // One 16-row block against all units: p[0..3] += scale * sums for (row0, col 2t), (row0, col 2t + 1), (row1, ...).
-// a_addr: this lane's ldmatrix row address for the block's first 32 bytes; sc: the 2 NG scales of rows row0, row0 + 1.
-template <int BITS, int UPG>
-__device__ __forceinline__ void block_pass(uint32_t a_addr, const unsigned short* sc, const uint32_t (&bf)[8],
+// a_addr: this lane's ldmatrix row address for the block's first 32 bytes; sc0, sc1: the NG scales of the two rows (SCALED), or not
+// looked at: the blocks of a state scaled along v carry no scale of their own.
+template <int BITS, int UPG, bool SCALED = true>
+__device__ __forceinline__ void block_pass(uint32_t a_addr, const unsigned short* sc0, const unsigned short* sc1, const uint32_t (&bf)[8],
                                            const int (&ci)[4 / UPG][2], float (&p)[4]) {
   constexpr int NG = 4 / UPG;
   float s0[NG], s1[NG];
-  if constexpr (NG == 4) {
-    const uint4 w = *reinterpret_cast<const uint4*>(sc);
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-    const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&w.z)), d = __half22float2(*reinterpret_cast<const __half2*>(&w.w));
-    s0[0] = a.x; s0[1] = a.y; s0[2] = b.x; s0[3] = b.y; s1[0] = c.x; s1[1] = c.y; s1[2] = d.x; s1[3] = d.y;
-  } else if constexpr (NG == 2) {
-    const uint2 w = *reinterpret_cast<const uint2*>(sc);
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-    s0[0] = a.x; s0[1] = a.y; s1[0] = b.x; s1[1] = b.y;
-  } else {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(sc);
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w));
-    s0[0] = a.x; s1[0] = a.y;
-  }
+  if constexpr (SCALED) { row_scales<NG>(sc0, s0); row_scales<NG>(sc1, s1); }
   int acc[NG][4];
 #pragma unroll
   for (int g = 0; g < NG; g++) { acc[g][0] = ci[g][0]; acc[g][1] = ci[g][1]; acc[g][2] = ci[g][0]; acc[g][3] = ci[g][1]; }
@@ -146,14 +164,14 @@ __device__ __forceinline__ void block_pass(uint32_t a_addr, const unsigned short
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       uint32_t m[4];
-      ldsm_x4(m, a_addr + 32 * j);
+      ldsm_x4(m, a_addr ^ (32 * j));
       mma_i8<false>(acc[j / UPG], m[0], m[1], m[2], m[3], bf[2 * j], bf[2 * j + 1]);
     }
   } else {
 #pragma unroll
     for (int J = 0; J < 2; J++) {
       uint32_t m[4];
-      ldsm_x4(m, a_addr + 32 * J);
+      ldsm_x4(m, a_addr ^ (32 * J));
       const uint32_t l0 = m[0] & 0x0F0F0F0Fu, l1 = m[1] & 0x0F0F0F0Fu, l2 = m[2] & 0x0F0F0F0Fu, l3 = m[3] & 0x0F0F0F0Fu;
       const uint32_t h0 = (m[0] >> 4) & 0x0F0F0F0Fu, h1 = (m[1] >> 4) & 0x0F0F0F0Fu, h2 = (m[2] >> 4) & 0x0F0F0F0Fu,
                      h3 = (m[3] >> 4) & 0x0F0F0F0Fu;
@@ -168,8 +186,13 @@ __device__ __forceinline__ void block_pass(uint32_t a_addr, const unsigned short
   for (int g = 0; g < NG; g++) {
     const float2 a01 = __fadd2_rn(make_float2(__int_as_float(acc[g][0]), __int_as_float(acc[g][1])), nm);
     const float2 a23 = __fadd2_rn(make_float2(__int_as_float(acc[g][2]), __int_as_float(acc[g][3])), nm);
-    p01 = __ffma2_rn(a01, make_float2(s0[g], s0[g]), p01);
-    p23 = __ffma2_rn(a23, make_float2(s1[g], s1[g]), p23);
+    if constexpr (SCALED) {
+      p01 = __ffma2_rn(a01, make_float2(s0[g], s0[g]), p01);
+      p23 = __ffma2_rn(a23, make_float2(s1[g], s1[g]), p23);
+    } else {
+      p01 = a01;
+      p23 = a23;
+    }
   }
   p[0] = p01.x; p[1] = p01.y; p[2] = p23.x; p[3] = p23.y;
 }
@@ -183,24 +206,20 @@ __device__ __forceinline__ float join_digits(const float (&p)[4], int t) {
   return ((t & 1) ? x1 : x0) + recv;
 }
 
-// The pass of one tile (32 rows = blocks 2w and 2w + 1 of a stage of 8 pieces): on return lane (i, t) holds the sums
-// of stage row i * R + 4 w + t against vector 0 (tq) and vector 1 (tk), in fixed-point units.
-// codes: shared address of the stage's first piece; pitch: bytes between pieces; scs: the stage's scales [row][NG].
-template <int BITS, int UPG, int R>
+// The pass of one tile (32 rows of a stage): on return lane (i, t) holds the sums of stage row tile_row(w, lane) against vector 0
+// (tq) and vector 1 (tk), in fixed-point units.  codes: shared address of the stage; scs: its scales [row][NG].
+template <int BITS, int UPG>
 __device__ __forceinline__ void tile_pass(uint32_t codes, const unsigned short* scs, const uint32_t (&bf)[8],
                                           const int (&ci)[4 / UPG][2], int w, int lane, float& tq, float& tk) {
   constexpr int NG = 4 / UPG;
-  constexpr int ROWB = 128 * BITS / 8;
-  constexpr int PITCH = R * ROWB + 16;
-  const int i = lane >> 2, t = lane & 3;
-  // ldmatrix: lane l gives the row address of matrix l / 8, row l % 8: piece l % 8, row 2b + (matrix & 1), byte half
-  const uint32_t lrow = codes + (lane & 7) * PITCH + ((lane >> 3) & 1) * ROWB + (lane >> 4) * 16;
+  const int t = lane & 3;
+  const uint32_t lrow = tile_lrow<BITS>(codes, w, lane, 0);
+  const unsigned short* sr = scs + (32 * w + (lane >> 2)) * NG;
   float T[2];
 #pragma unroll
   for (int bb = 0; bb < 2; bb++) {
-    const int b = 2 * w + bb;
     float p[4] = {0.f, 0.f, 0.f, 0.f};
-    block_pass<BITS, UPG>(lrow + 2 * b * ROWB, scs + (i * R + 2 * b) * NG, bf, ci, p);
+    block_pass<BITS, UPG>(lrow + bb * 16 * (128 * BITS / 8), sr + bb * 16 * NG, sr + (bb * 16 + 8) * NG, bf, ci, p);
     T[bb] = join_digits(p, t);
   }
   const float recv = __shfl_xor_sync(0xffffffffu, t < 2 ? T[1] : T[0], 2);
@@ -210,33 +229,8 @@ __device__ __forceinline__ void tile_pass(uint32_t codes, const unsigned short* 
 
 // ---- states scaled along v (one scale per column for every group of 32 rows) ------------------------------------------
 // The scale varies along the contraction, so it goes into the read-out vectors: group G of a head is read against
-// q * scale_G and k * scale_G, in fixed point as above, and the integer sums need no scale afterwards.  A warp takes
-// exactly one group: rows 32 w .. 32 w + 31 of the stage = pieces 2w and 2w + 1, and builds its own B fragments for it.
-// Block bb (16 rows): fragment row f = row (f >> 1) + 8 bb of piece 2w + (f & 1).  With 64-byte rows (4-bit codes) the
-// eight row addresses of an ldmatrix tile then fall on four distinct 16-byte bank groups (a two-way conflict); with
-// 128-byte rows they would all collide, so 8-bit codes scaled along v are staged in smaller pieces (below).
-// On return lane (i, t) holds the sums of stage row 32 w + 16 (i & 1) + (i >> 1) + 4 (t & 1) + 8 (t >> 1).
-
-// 8-bit codes (128-byte rows) scaled along v come in 32 pieces of FOUR rows instead (pitch 4 * 128 + 16): a group is
-// then eight pieces, fragment row i < 8 is row 2 bb of piece 8 w + i and fragment row 8 + i its row 2 bb + 1, and the
-// eight row addresses of an ldmatrix tile fall on distinct banks again.  On return lane (i, t) holds stage row
-// 32 w + 4 i + t.
-constexpr int V8_PIECE_ROWS = 4, V8_PITCH = V8_PIECE_ROWS * 128 + 16;
-
-// This lane's stage row in the layouts above.
-template <int BITS>
-__device__ __forceinline__ int tile_row_v(int w, int lane) {
-  const int i = lane >> 2, t = lane & 3;
-  if (BITS == 8) return 32 * w + 4 * i + t;
-  return 32 * w + 16 * (i & 1) + (i >> 1) + 4 * (t & 1) + 8 * (t >> 1);
-}
-// shared address of the ldmatrix row this lane supplies for block bb of warp w's group (first 32 bytes of the rows)
-template <int BITS>
-__device__ __forceinline__ uint32_t tile_lrow_v(uint32_t codes, int w, int lane, int bb) {
-  if (BITS == 8) return codes + (8 * w + (lane & 7)) * V8_PITCH + (2 * bb + ((lane >> 3) & 1)) * 128 + (lane >> 4) * 16;
-  constexpr int ROWB = 64, PITCH = 16 * ROWB + 16;
-  return codes + (2 * w + (lane & 1)) * PITCH + (((lane & 7) >> 1) + 4 * ((lane >> 3) & 1) + 8 * bb) * ROWB + (lane >> 4) * 16;
-}
+// q * scale_G and k * scale_G, in fixed point as above, and the integer sums need no scale afterwards.  A warp's 32 rows are
+// exactly one group, and it builds its own B fragments for it.
 
 // The warp's B fragments for its group: sg = the group's 128 column scales (fp16), vq / vk = the read-out vectors
 // (fp32, 128 each; vk unused if !TWO).  Bf: the warp's own 1 KB of shared memory.  Returns the fixed-point scales.
@@ -269,18 +263,17 @@ __device__ __forceinline__ void build_b_v(uint32_t* Bf, const unsigned short* sg
   for (int r = 0; r < 8; r++) bf[r] = Bf[r * 32 + lane];
 }
 
-// one: shared address of a word holding the fp16 pair (1, 1) (the blocks carry no scale of their own)
 template <int BITS>
-__device__ __forceinline__ void tile_pass_v(uint32_t codes, const unsigned short* one, const uint32_t (&bf)[8], int w,
-                                            int lane, float& tq, float& tk) {
+__device__ __forceinline__ void tile_pass_v(uint32_t codes, const uint32_t (&bf)[8], int w, int lane, float& tq, float& tk) {
   const int t = lane & 3;
   int ci[1][2];
   acc_start<BITS, 4>(bf, ci);
+  const uint32_t lrow = tile_lrow<BITS>(codes, w, lane, 0);
   float T[2];
 #pragma unroll
   for (int bb = 0; bb < 2; bb++) {
     float p[4] = {0.f, 0.f, 0.f, 0.f};
-    block_pass<BITS, 4>(tile_lrow_v<BITS>(codes, w, lane, bb), one, bf, ci, p);
+    block_pass<BITS, 4, false>(lrow + bb * 16 * (128 * BITS / 8), nullptr, nullptr, bf, ci, p);
     T[bb] = join_digits(p, t);
   }
   const float recv = __shfl_xor_sync(0xffffffffu, t < 2 ? T[1] : T[0], 2);

@@ -56,14 +56,12 @@ __host__ __device__ inline SmemM smemm_plan(int kind, int bits, int upg, int DV,
   const bool simt = fold && !fold_on_tensor_pipe(kind, bits, upg, M, axv), tens = fold && !simt;
   SmemM s;
   const int rowb = 128 * bits / 8, ng = 4 / upg;
-  const bool v8 = axv && bits == 8;                  // 8-bit codes scaled along v: 32 pieces of 4 rows (mma_pass.cuh)
-  const int pitch = v8 ? V8_PITCH : 16 * rowb + 16;
-  s.sc_off = (v8 ? 32 : 8) * pitch;
+  s.sc_off = 128 * rowb;
   s.ub_off = s.sc_off + 128 * ng * 2;
-  s.stage_bytes = s.ub_off + al16i(M * 128);
+  s.stage_bytes = (s.ub_off + al16i(M * 128) + 1023) & ~1023;       // (the swizzle repeats every 1024 bytes)
   int o = 0;
-  s.bars = o; o += 128;
   s.stage0 = o; o += nst * s.stage_bytes;
+  s.bars = o; o += 128;
   s.kb = o; o += al16i(M * 128);
   s.gbt = o; o += (kind == K_KDA ? M * 128 * 4 : 0);
   s.bf = o; o += (bits == 4 && kind != K_KDA) ? 2048 : 1024;   // B fragments: the state's layout (+ the byte layout for the key tile)
@@ -134,20 +132,20 @@ static __device__ __noinline__ void mma_bail(uint8_t* orow, int dt, int n, uint6
 template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV = false, bool BIO = false>
 __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((BITS == 8 && UPG == 1) || (BITS == 4 && UPG == 2)) ? SQB_MMA_MINB_TFOLD : SQB_MMA_MINB_FOLD))
                                                : (BITS == 4 ? SQB_MMA_MINB4 : SQB_MMA_MINB8))
-    step_mma_kernel(const __grid_constant__ StepArgs A, const __grid_constant__ SmemM P, const int nst) {
+    step_mma_kernel(const __grid_constant__ StepArgs A, const __grid_constant__ TileMap codes_map, const __grid_constant__ SmemM P,
+                    const int nst) {
   dependency_wait();
   dependency_release();
   constexpr int DK = 128, NG = 4 / UPG, G = 32 * UPG;
-  constexpr bool V8 = AXV && BITS == 8;          // 32 pieces of 4 rows instead of 8 pieces of 16
-  constexpr int ROWB = DK * BITS / 8, PROWS = V8 ? V8_PIECE_ROWS : 16, PITCH = PROWS * ROWB + 16;
-  constexpr int HPS = 128 / DV;                  // heads per stage
+  constexpr int ROWB = DK * BITS / 8;
+  constexpr int HPS = 128 / DV, WPH = 4 / HPS;   // heads per stage, warps per head (a head's maxima are kept 4 / WPH times over)
   constexpr int CW = 4;                          // columns per lane in the prologue
   constexpr bool TWO = KIND != K_M2, VDEC = KIND == K_KDA, CANFOLD = MODE == 3;
   constexpr bool TFMT = AXV || (BITS == 8 && UPG == 1) || (BITS == 4 && UPG == 2);
   static_assert(DV == 64 || DV == 128, "a stage is 128 rows: one or two heads");
   static_assert(!AXV || (UPG == 1 && !VDEC), "scales along v: groups of 32 rows (the stage's scales are [4][128], as many bytes as UPG = 1)");
 
-  extern __shared__ __align__(128) uint8_t smraw[];
+  extern __shared__ __align__(1024) uint8_t smraw[];
   const int dt_qk = BIO ? static_cast<int>(DT_BF16) : A.dt_qk, dt_v = BIO ? static_cast<int>(DT_BF16) : A.dt_v,
             dt_out = BIO ? static_cast<int>(DT_BF16) : A.dt_out;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -176,7 +174,7 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
   // a loaded word already waits for it), and a wait never sits in front of fetches that do not depend on it:
   //   warps 0 and 3 need q and k first and the slot only later: their q / k loads leave before the slot index;
   //   warps 1 and 2 issue the bulk copies, which need nothing but the slot index: they load it alone.
-  const int rho = AXV ? tile_row_v<BITS>(warp, lane) : (lane >> 2) * 16 + 4 * warp + (lane & 3);     // this lane's row within a stage
+  const int rho = tile_row(warp, lane);                          // this lane's row within a stage
   const int hh = rho / DV, rv = rho % DV;                        // head within the stage, row within the head
   Raw4 rq, rk;
   rq.v = make_uint4(0u, 0u, 0u, 0u); rk.v = rq.v; rq.vec = false; rk.vec = false;
@@ -224,19 +222,13 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     gck = *reinterpret_cast<const float4*>(GCseq + (long long)h0 * DK + lane * CW);
   }
 
-  // the copies of stage `sh` into ring position s, one per lane (lanes 0..9 of the calling warp)
+  // the copies of stage `sh` into ring position s, one per lane (lanes 0 .. 2 of the calling warp)
   auto issue_stage = [&](int s, int sh, int l) {
     uint8_t* st = smraw + P.stage0 + s * P.stage_bytes;
     const long long row0 = (long long)h0 * DV + sh * 128;
-    if constexpr (V8) {                                      // 32 pieces take every lane: two of them copy twice
-      bulk_g2s(st + l * PITCH, Sseq + (row0 + l * PROWS) * ROWB, PROWS * ROWB, &bars[s]);
-      if (l == 0) bulk_g2s(st + P.sc_off, SCseq + row0 * NG * 2, 128 * NG * 2, &bars[s]);
-      else if (l == 1) bulk_g2s(st + P.ub_off, UBseq + (long long)(h0 + sh * HPS) * M * DV, M * 128, &bars[s]);
-    } else {
-      if (l < 8) bulk_g2s(st + l * PITCH, Sseq + (row0 + l * 16) * ROWB, 16 * ROWB, &bars[s]);
-      else if (l == 8) bulk_g2s(st + P.sc_off, SCseq + row0 * NG * 2, 128 * NG * 2, &bars[s]);
-      else if (l == 9) bulk_g2s(st + P.ub_off, UBseq + (long long)(h0 + sh * HPS) * M * DV, M * 128, &bars[s]);
-    }
+    if (l == 0) tile_g2s(st, &codes_map, static_cast<int>(row0), static_cast<int>(seq), &bars[s]);
+    else if (l == 1) bulk_g2s(st + P.sc_off, SCseq + row0 * NG * 2, 128 * NG * 2, &bars[s]);
+    else if (l == 2) bulk_g2s(st + P.ub_off, UBseq + (long long)(h0 + sh * HPS) * M * DV, M * 128, &bars[s]);
   };
   // A stage barrier of the first fill is initialised, armed and its copies issued by ONE warp (a warp's copies leave
   // one after the other, so the stages are spread over warps 2 and 1); everybody else meets it after the block barrier.
@@ -446,7 +438,6 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     if constexpr (AXV) {                    // every warp scales the vectors by its group's column scales, per stage
       *reinterpret_cast<float4*>(wq + lane * CW) = make_float4(eq[0], eq[1], eq[2], eq[3]);
       *reinterpret_cast<float4*>(wk + lane * CW) = make_float4(ek[0], ek[1], ek[2], ek[3]);
-      if (lane == 0) misc[9] = __uint_as_float(0x3C003C00u);      // the fp16 pair (1, 1): the blocks carry no scale
       if (BITS == 8) {                      // the key tile's product still takes the plain vectors, in the byte layout
         put_b_words<8>(Bfw, lane, 0, yq[0], yq[1], yq[2], yq[3]);
         put_b_words<8>(Bfw, lane, 1, yk[0], yk[1], yk[2], yk[3]);
@@ -676,16 +667,15 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
         uint32_t bfB[8];
         FxScale fqA, fkA, fqB, fkB;
         uint32_t* area = reinterpret_cast<uint32_t*>(smraw + P.bfv) + warp * 256;
-        const unsigned short* one = reinterpret_cast<const unsigned short*>(misc + 9);
         build_b_v<BITS, TWO>(area, reinterpret_cast<const unsigned short*>(stA + P.sc_off) + warp * 128, wq, wk, lane, bf, fqA, fkA);
         build_b_v<BITS, TWO>(area, reinterpret_cast<const unsigned short*>(stB + P.sc_off) + warp * 128, wq, wk, lane, bfB, fqB, fkB);
-        tile_pass_v<BITS>(smem_u32(stA), one, bf, warp, lane, tqA, tkA);
-        tile_pass_v<BITS>(smem_u32(stB), one, bfB, warp, lane, tqB, tkB);
+        tile_pass_v<BITS>(smem_u32(stA), bf, warp, lane, tqA, tkA);
+        tile_pass_v<BITS>(smem_u32(stB), bfB, warp, lane, tqB, tkB);
         tqA = (tqA * fqA.i1) * fqA.i2; tqB = (tqB * fqB.i1) * fqB.i2;
         if (TWO) { tkA = (tkA * fkA.i1) * fkA.i2; tkB = (tkB * fkB.i1) * fkB.i2; }
       } else {
-        tile_pass<BITS, UPG, 16>(smem_u32(stA), reinterpret_cast<const unsigned short*>(stA + P.sc_off), bf, ci, warp, lane, tqA, tkA);
-        tile_pass<BITS, UPG, 16>(smem_u32(stB), reinterpret_cast<const unsigned short*>(stB + P.sc_off), bf, ci, warp, lane, tqB, tkB);
+        tile_pass<BITS, UPG>(smem_u32(stA), reinterpret_cast<const unsigned short*>(stA + P.sc_off), bf, ci, warp, lane, tqA, tkA);
+        tile_pass<BITS, UPG>(smem_u32(stB), reinterpret_cast<const unsigned short*>(stB + P.sc_off), bf, ci, warp, lane, tqB, tkB);
         tqA = (tqA * iq1) * iq2; tqB = (tqB * iq1) * iq2;       // powers of two: exact
         if (TWO) { tkA = (tkA * ik1) * ik2; tkB = (tkB * ik1) * ik2; }
       }
@@ -718,10 +708,9 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       uint8_t* orow = A.out + (long long)b * A.so + (long long)(h0 + hiA) * DV * osz;
       stf(orow, dt_out, rv, oA);
       stf(orow + (long long)HPS * DV * osz, dt_out, rv, oB);
-      const uint32_t umask = HPS == 1 ? 0xffffffffu : (lane < 16 ? 0x0000ffffu : 0xffff0000u);
-      const float mA = __uint_as_float(__reduce_max_sync(umask, __float_as_uint(fabsf(uA))));
-      const float mB = __uint_as_float(__reduce_max_sync(umask, __float_as_uint(fabsf(uB))));
-      if ((lane & (HPS == 1 ? 31 : 15)) == 0) { red[hiA * NW + warp] = mA; red[hiB * NW + warp] = mB; }
+      const float mA = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(uA))));
+      const float mB = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(uB))));
+      if (lane < 4 / WPH) { red[hiA * NW + warp % WPH + lane * WPH] = mA; red[hiB * NW + warp % WPH + lane * WPH] = mB; }
     }
   } else
   for (int sh = 0; sh < NSH; sh++) {
@@ -744,11 +733,11 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     if constexpr (AXV) {
       FxScale fq, fk;
       build_b_v<BITS, TWO>(reinterpret_cast<uint32_t*>(smraw + P.bfv) + warp * 256, scs + warp * 128, wq, wk, lane, bf, fq, fk);
-      tile_pass_v<BITS>(smem_u32(st), reinterpret_cast<const unsigned short*>(misc + 9), bf, warp, lane, tq, tk);
+      tile_pass_v<BITS>(smem_u32(st), bf, warp, lane, tq, tk);
       tq = (tq * fq.i1) * fq.i2;
       if (TWO) tk = (tk * fk.i1) * fk.i2;
     } else {
-      tile_pass<BITS, UPG, 16>(smem_u32(st), scs, bf, ci, warp, lane, tq, tk);
+      tile_pass<BITS, UPG>(smem_u32(st), scs, bf, ci, warp, lane, tq, tk);
       tq = (tq * iq1) * iq2;                                  // powers of two: exact
       if (TWO) tk = (tk * ik1) * ik2;
     }
@@ -777,9 +766,8 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     stf(A.out + (long long)b * A.so + (long long)h * DV * osz, dt_out, rv, o);
     // largest |u| of the head's rows in this warp: non-negative floats order like their bit patterns (a NaN ends up
     // as the maximum, as it should)
-    const uint32_t umask = HPS == 1 ? 0xffffffffu : (lane < 16 ? 0x0000ffffu : 0xffff0000u);
-    const float umax = __uint_as_float(__reduce_max_sync(umask, __float_as_uint(fabsf(u))));
-    if ((lane & (HPS == 1 ? 31 : 15)) == 0) red[hi * NW + warp] = umax;
+    const float umax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(u))));
+    if (lane < 4 / WPH) red[hi * NW + warp % WPH + lane * WPH] = umax;
     SQB_STAMP(7 + 3 * (sh & 1));
 
     if (CANFOLD && FOLD) {
@@ -827,18 +815,13 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
             fold_stage_mma<BITS, UPG, DV, VDEC>(smem_u32(st), reinterpret_cast<unsigned short*>(st + P.sc_off),
                                                 reinterpret_cast<const int8_t*>(st + P.ub_off), us + sh * HPS * DV, tab, ksf, KBf,
                                                 warp, lane, ae);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncthreads();
           if (warp == 0) {
-            // the stage goes back to the slot: eight pieces of codes and the scales, as bulk copies
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            // the stage goes back to the slot: codes and scales, a copy each
             const long long row0 = (long long)h0 * DV + sh * 128;
-            if constexpr (V8) {
-              bulk_s2g(Sseq + (row0 + lane * PROWS) * ROWB, st + lane * PITCH, PROWS * ROWB);
-              if (lane == 0) bulk_s2g(SCseq + row0 * NG * 2, st + P.sc_off, 128 * NG * 2);
-            } else {
-              if (lane < 8) bulk_s2g(Sseq + (row0 + lane * 16) * ROWB, st + lane * PITCH, 16 * ROWB);
-              else if (lane == 8) bulk_s2g(SCseq + row0 * NG * 2, st + P.sc_off, 128 * NG * 2);
-            }
+            if (lane == 0) tile_s2g(&codes_map, static_cast<int>(row0), static_cast<int>(seq), st);
+            else if (lane == 1) bulk_s2g(SCseq + row0 * NG * 2, st + P.sc_off, 128 * NG * 2);
             bulk_commit();
             if (sh + nst < NSH || sh + 1 == NSH) bulk_wait_read();   // before the stage is refilled, and before leaving
           }
@@ -878,7 +861,7 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
         }
         __syncthreads();
         const float alphan = VDEC ? 1.0f : expf(gnew);
-        fold_rows<BITS, true, 8, VDEC, true>(st + hq * (DV / 16) * PITCH,
+        fold_rows<BITS, true, 8, VDEC, true>(st + hq * DV * ROWB,
                                              reinterpret_cast<const unsigned short*>(st + P.sc_off) + hq * DV * NG, Rf, Lf, ae,
                                              alphan, DV, G, M, nullptr, Sseq + (long long)hg * DV * ROWB,
                                              reinterpret_cast<unsigned short*>(SCseq) + (long long)hg * DV * NG, warp, lane, tid,
