@@ -55,13 +55,15 @@ __device__ __forceinline__ float cvt_raw(uint32_t w, int dt) {
 }
 // Elements i .. i + 3 (i a multiple of 4) as loaded, untouched: unpacking a loaded word is already a use that waits
 // for the load, so it is left to cvt4_raw.  vec: the row is read by one 8- or 16-byte load (the address allows it).
+// ALIGNED: the caller knows that it does.
 struct Raw4 { uint4 v; bool vec; };
+template <bool ALIGNED = false>
 __device__ __forceinline__ Raw4 ld4_raw(const uint8_t* p, int dt, long long i) {
   Raw4 r;
   r.v = make_uint4(0u, 0u, 0u, 0u);
   if (dt == DT_F32) {
     const uint8_t* q = p + 4 * i;
-    r.vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+    r.vec = ALIGNED || (reinterpret_cast<uintptr_t>(q) & 15) == 0;
     if (r.vec) {
       r.v = *reinterpret_cast<const uint4*>(q);
     } else {
@@ -70,7 +72,7 @@ __device__ __forceinline__ Raw4 ld4_raw(const uint8_t* p, int dt, long long i) {
     }
   } else {
     const uint8_t* q = p + 2 * i;
-    r.vec = (reinterpret_cast<uintptr_t>(q) & 7) == 0;
+    r.vec = ALIGNED || (reinterpret_cast<uintptr_t>(q) & 7) == 0;
     if (r.vec) {
       const uint2 t = *reinterpret_cast<const uint2*>(q);
       r.v.x = t.x; r.v.y = t.y;
@@ -81,8 +83,9 @@ __device__ __forceinline__ Raw4 ld4_raw(const uint8_t* p, int dt, long long i) {
   }
   return r;
 }
+template <bool ALIGNED = false>
 __device__ __forceinline__ void cvt4_raw(const Raw4& r, int dt, float (&f)[4]) {
-  if (dt == DT_F32 || !r.vec) {
+  if (dt == DT_F32 || !(ALIGNED || r.vec)) {
     f[0] = cvt_raw(r.v.x, dt); f[1] = cvt_raw(r.v.y, dt); f[2] = cvt_raw(r.v.z, dt); f[3] = cvt_raw(r.v.w, dt);
   } else {
     f[0] = cvt_raw(r.v.x & 0xFFFFu, dt); f[1] = cvt_raw(r.v.x >> 16, dt);
@@ -98,17 +101,19 @@ __device__ __forceinline__ unsigned short f2bf(float f) { return __bfloat16_as_u
 // Quantizer scale of a group with absolute maximum amax (see the contract above).
 // x / qmax for the two code ranges in use, without the division: with r = RN(1 / qmax), q0 = RN(x r),
 // q = fma(fma(-qmax, q0, x), r, q0) equals div_rn(x, qmax) for EVERY finite float x in [1e-8, 3e38] when qmax is 127
-// or 7 (checked exhaustively on the host, tests/div_const_check.c); anything else takes the IEEE division.
+// or 7 (checked exhaustively on the host, tests/div_const_check.c); x is in that range, and other divisors take the IEEE division.
 __device__ __forceinline__ float div_qmax(float x, float qmax) {
-  if ((qmax == 127.0f || qmax == 7.0f) && x <= 3.0e38f) {
+  if (qmax == 127.0f || qmax == 7.0f) {
     const float r = qmax == 127.0f ? 0x1.020408p-7f : 0x1.24924ap-3f;
     const float q0 = __fmul_rn(x, r);
     return __fmaf_rn(__fmaf_rn(-qmax, q0, x), r, q0);
   }
   return __fdiv_rn(x, qmax);
 }
+// (A maximum beyond 3e38 gives fp16's infinity like 3e38 does, so no code for the division of such a one is carried; a NaN counts
+// as 1e-8.)
 __device__ __forceinline__ float fp16_scale(float amax, float qmax) {
-  float s = div_qmax(fmaxf(amax, 1e-8f), qmax);
+  float s = div_qmax(fminf(fmaxf(amax, 1e-8f), 3.0e38f), qmax);
   s = h2f(f2h(s));
   return fmaxf(s, FP16_TINY);
 }
@@ -121,6 +126,40 @@ __device__ __forceinline__ float rcp_approx(float s) {
 // clamp(rint(x / s), +-qmax), exact
 __device__ __forceinline__ float rq_exact(float x, float s, float qmax) {
   return fminf(fmaxf(rintf(__fdiv_rn(x, s)), -qmax), qmax);
+}
+
+// clamp(rint(x / s), +-127) by the IEEE division: the rare exact path of a buffer entry's rounding
+static __device__ __noinline__ float rq_exact_cold(float x, float s) { return rq_exact(x, s, 127.0f); }
+// clamp(rint(x / s), +-127) of four values, s the scale of a vector that holds them: by the reciprocal, verified, and by the division
+// next to a tie or where the scale lies far from the maximum / 127
+__device__ __forceinline__ void round4(const float (&x)[4], float s, float (&c)[4]) {
+  const float r = rcp_approx(s);
+  bool near = s < FP16_MIN_NORMAL;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    c[j] = fmaf(x[j], r, MAGIC) - MAGIC;
+    near |= !(fabsf(fmaf(-c[j], s, x[j])) < s * 0.49998474f);
+  }
+  if (near) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) c[j] = rq_exact_cold(x[j], s);
+  }
+}
+// x[j] / s, s the norm of a vector that holds the x: correctly rounded (Markstein: the reciprocal is, and the residual is exact)
+// but for quotients below 2^-100, which end up as code 0 either way.  A norm near the top of the range takes the division.
+static __device__ __noinline__ float div_cold(float x, float s) { return __fdiv_rn(x, s); }
+__device__ __forceinline__ void div_norm(float (&x)[4], float s) {
+  if (s < 1e37f) {
+    const float r = __frcp_rn(s);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float q = x[j] * r;
+      x[j] = fmaf(fmaf(-s, q, x[j]), r, q);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; j++) x[j] = div_cold(x[j], s);
+  }
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

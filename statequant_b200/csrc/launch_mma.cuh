@@ -63,10 +63,10 @@ inline bool mma_plan(const StepArgs& a, int bits, int mode, SmemM& plan, int& ns
 template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV, bool BIO>
 int launch_mma_one_io(const StepArgs& a, cudaStream_t stream);
 
-// bf16 activations and output take the kernel with those element types compiled in
+// bf16 activations and output (bf16_io) take the kernel with those element types compiled in
 template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV = false>
 int launch_mma_one(const StepArgs& a, cudaStream_t stream) {
-  if (a.dt_qk == DT_BF16 && a.dt_v == DT_BF16 && a.dt_out == DT_BF16)
+  if (bf16_io(a))
     return launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, true>(a, stream);
   return launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, false>(a, stream);
 }

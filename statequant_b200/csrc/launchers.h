@@ -75,6 +75,12 @@ struct Residency {
 // wave where slots are due one in eight: 608 CTAs 12.1 / 12.9, 736 12.8 / 13.4 (all due 7.8 / 7.6, 8.3 / 7.8), 1024 17.6 / 17.4.
 inline bool enters_early(long long grid, long long all, bool kda) { return 2 * grid <= all || (kda ? grid > all : 5 * grid > 4 * all); }
 
+// bf16 activations and output with q and k rows on 8-byte boundaries: the step kernels have instances of their own for these.
+inline bool bf16_io(const StepArgs& a) {
+  return a.dt_qk == DT_BF16 && a.dt_v == DT_BF16 && a.dt_out == DT_BF16 &&
+         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | static_cast<uintptr_t>(a.sq) | static_cast<uintptr_t>(a.sk)) & 7) == 0;
+}
+
 // Shapes the register-tile step takes: d_k 128 and d_v 64 or 128 with bf16 states or (Gated DeltaNet, Mamba2) 8-bit codes in
 // key groups of 32 or 4-bit codes in key groups of 64; Gated DeltaNet states of d_k 96 and d_v 64, 128 or 192 with those codes;
 // decays per head, int8 buffer of 8, q / k per key head, a CTA's rows of one key head.

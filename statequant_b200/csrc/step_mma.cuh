@@ -3,11 +3,11 @@
 // d_v 64 or 128, int8 decode buffer.
 //
 // One CTA (128 threads) per (batch row, KEY head, part of its value heads) walks its value heads in STAGES of 128
-// state rows (one head of d_v 128, two heads of d_v 64).  A stage -- codes as 8 padded pieces, scales, buffered
+// state rows (one head of d_v 128, two heads of d_v 64).  A stage -- codes (swizzled), scales, buffered
 // values -- arrives by bulk async copies on one mbarrier; the copies of the first stages and of the key tile are
 // issued by the lanes of warps 2 and 1 in the CTA's first instructions.  Per stage each warp takes a tile of 32 rows
 // through the tensor-core pass and finishes one row per lane (buffer term, u, o).  A CTA with exactly two stages takes
-// both at once on a token that does not fold: two independent chains per warp instead of one after the other.
+// both at once: two independent chains per warp instead of one after the other.
 //
 // MODE 0: every token is stepped and appended (after the last stage); on a slot's m-th token the head's counter is
 //         left at m for the fold launch that follows (fold_kernel.cuh).
@@ -17,11 +17,19 @@
 //         Nothing a CTA fetches depends on the slot's counter, so every copy and every scalar load leaves in the
 //         CTA's first instructions.
 //
-// Prologue by role: warp 0 normalises q and k, builds the fixed-point B fragments and (GDN, Mamba2) takes the
-// buffered keys' dot products on the tensor pipe; warp 1 the gates; warp 2 issues the copies and computes decay
-// factors and value scales of every (head, slot); warp 3 rounds the key that goes into the buffer (KDA: prepares the
-// normalised vectors and log decays for the buffered keys' products, which all four warps take in fp32 after the
-// block barrier, their decay ratios being per channel; warp 0 rounds the key).
+// Prologue by role: warp 0 builds the fixed-point B fragments of q and k and (GDN, Mamba2) takes the buffered keys' dot products
+// on the tensor pipe; warp 1 the gates; warp 2 issues the copies and computes decay factors and value scales of every (head, slot);
+// warp 3 rounds the key that goes into the buffer and, decays per head, finds the vectors' norms, which are applied to the finished
+// sums (KDA: prepares the normalised vectors and log decays for the buffered keys' products, which all four warps take in fp32
+// after the block barrier, their decay ratios being per channel; warp 0 rounds the key).  (k on a warp of its own, gates and decays
+// on another: 3 % slower, int8 k/32 256 rows 40.7 -> 42.0 us.)
+//
+// Long grids are bound by instruction issue and fetch: a CTA's warps walk 1000 instructions each that nothing repeats, out of a
+// kernel of 60 .. 90 KB, and CTAs that fold want other code than those that do not.  So a token that folds goes through the same
+// read-out and append as one that does not, and what serves no ordinary call is kept out of line.  int4 k/64, 1024 rows with a slot in
+// eight folding: 207 -> 171 us, cycles a warp waits for an instruction per instruction issued 3.1 -> 2.2; us per layer-step at 256 rows,
+// all slots on one token / each on its own: int8 k/32 44.1 -> 40.7 / 57.2 -> 48.0, int4 k/64 43.7 -> 38.9 / 56.7 -> 48.2, Mamba2 int8 78.9
+// -> 73.4 / 97.5 -> 79.8, int4 v/32 (192 rows) 40.3 -> 36.8 / 52.9 -> 45.3.
 //
 // Arithmetic is that of delta_step.cuh (same rounding of scales, payloads and buffer entries); only the order of the
 // reductions differs, and the read-out vectors pass through 30-bit fixed point (mma_pass.cuh).
@@ -84,7 +92,7 @@ __host__ __device__ inline SmemM smemm_plan(int kind, int bits, int upg, int DV,
   s.wk = f; f += (kind == K_KDA || axv ? 128 : 0);
   s.wg = f; f += (kind == K_KDA ? 128 : 0);
   f = (f + 3) & ~3;
-  s.tab = f; f += tens ? 2 * 20 : 0;
+  s.tab = f; f += tens ? 4 * 20 : 0;                   // (two stages of two heads)
   s.R = f; f += simt ? M * 160 : 0;
   s.L = f; f += simt ? DV * fold_lm(M) : 0;
   s.fdec = f; f += simt ? 32 : 0;
@@ -112,8 +120,6 @@ __host__ __device__ inline SmemM smemm_plan(int kind, int bits, int upg, int DV,
 
 // Cold paths kept out of line (they are never taken in a healthy run, and inlined at every use they were an eighth of
 // the kernel's code): the zero fill of a CTA's output rows, and the exit of a CTA whose copy never completed.
-// clamp(rint(x / s), +-127) by the IEEE division: the rare exact path of a buffer entry's rounding
-static __device__ __noinline__ float rq_exact_cold(float x, float s) { return rq_exact(x, s, 127.0f); }
 static __device__ __noinline__ void zero_out_rows(uint8_t* orow, int dt, int n) {
   for (int v = threadIdx.x; v < n; v += NT) stf(orow, dt, v, 0.0f);
 }
@@ -127,7 +133,7 @@ static __device__ __noinline__ void mma_bail(uint8_t* orow, int dt, int n, uint6
   }
 }
 
-// BIO: q / k / v and the output are bf16 (what a serving engine passes): the element types of the activation loads and
+// BIO: q / k / v and the output are bf16, q and k on 8-byte boundaries (what a serving engine passes): the element types of the activation loads and
 // stores are then compile-time constants instead of three-way run-time dispatches at every access.
 template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV = false, bool BIO = false>
 __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((BITS == 8 && UPG == 1) || (BITS == 4 && UPG == 2)) ? SQB_MMA_MINB_TFOLD : SQB_MMA_MINB_FOLD))
@@ -179,8 +185,8 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
   Raw4 rq, rk;
   rq.v = make_uint4(0u, 0u, 0u, 0u); rk.v = rq.v; rq.vec = false; rk.vec = false;
   if (warp == 0 || warp == 3) {
-    rq = ld4_raw(A.q + (long long)b * A.sq, dt_qk, (long long)hk * DK + lane * CW);
-    rk = ld4_raw(A.k + (long long)b * A.sk, dt_qk, (long long)hk * DK + lane * CW);
+    rq = ld4_raw<BIO>(A.q + (long long)b * A.sq, dt_qk, (long long)hk * DK + lane * CW);
+    rk = ld4_raw<BIO>(A.k + (long long)b * A.sk, dt_qk, (long long)hk * DK + lane * CW);
   }
   long long seq = b;
   if (A.idx != nullptr) {
@@ -260,11 +266,12 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
   float kdeq[CW] = {0.f, 0.f, 0.f, 0.f};
   auto round_key = [&](const float (&kr)[CW], float mx) {
     kscale = fp16_scale(mx, 127.0f);
+    float cc[CW];
+    round4(kr, kscale, cc);
 #pragma unroll
     for (int j = 0; j < CW; j++) {
-      const float cc = rq_exact(kr[j], kscale, 127.0f);
-      kword |= (static_cast<uint32_t>(static_cast<int>(cc)) & 0xFFu) << (8 * j);
-      kdeq[j] = cc * kscale;
+      kword |= (static_cast<uint32_t>(static_cast<int>(cc[j])) & 0xFFu) << (8 * j);
+      kdeq[j] = cc[j] * kscale;
     }
   };
 
@@ -384,8 +391,8 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     // pipe; KDA: the key that goes into the buffer
     load_v();
     float qr[CW], kr[CW];
-    cvt4_raw(rq, dt_qk, qr);
-    cvt4_raw(rk, dt_qk, kr);
+    cvt4_raw<BIO>(rq, dt_qk, qr);
+    cvt4_raw<BIO>(rk, dt_qk, kr);
     float gnr[CW] = {0.f, 0.f, 0.f, 0.f};
     float s0 = 0.f, s1 = 0.f;
     if constexpr (VDEC) {
@@ -399,7 +406,7 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       s1 += kr[j] * kr[j];
     }
     SQB_STAMP(1);
-    if (KIND != K_M2) {
+    if constexpr (VDEC) {
       s0 = warp_sum(s0);
       s1 = warp_sum(s1);
       const float nq = __fsqrt_rn(s0 + 1e-6f), nk = __fsqrt_rn(s1 + 1e-6f);
@@ -409,12 +416,14 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
         kr[j] = __fdiv_rn(kr[j], nk);
       }
     }
+    // Decays per head: q and k as they come; what their norms make of the sums every row applies at the end (warp 3 finds the
+    // factors meanwhile).
     float d = 0.f, mx = 0.f;
     float eq[CW], ek[CW], mq = 0.f, mk = 0.f;              // the vectors the state is read against
 #pragma unroll
     for (int j = 0; j < CW; j++) {
-      d += kr[j] * qr[j];
-      mx = fmaxf(mx, fabsf(kr[j]));
+      if (VDEC || KIND == K_M2) d += kr[j] * qr[j];
+      if (VDEC) mx = fmaxf(mx, fabsf(kr[j]));
       eq[j] = qr[j];
       ek[j] = kr[j];
       if (VDEC) {
@@ -429,12 +438,16 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     }
     // maxima of non-negative floats: their bit patterns order like integers (one reduction instruction each)
     mq = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mq)));
-    if (TWO && VDEC) mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
-    if (TWO && !VDEC) { mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx))); mk = mx; }
+    if (TWO) mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
     const FxScale fq = fx30_scale(mq), fk = fx30_scale(mk);
     uint32_t yq[CW], yk[CW];
 #pragma unroll
-    for (int j = 0; j < CW; j++) { yq[j] = fx30_digits(eq[j], fq); yk[j] = TWO ? fx30_digits(ek[j], fk) : 0u; }
+    for (int j = 0; j < CW; j++) {
+      eq[j] = (eq[j] * fq.m1) * fq.m2;
+      if (TWO) ek[j] = (ek[j] * fk.m1) * fk.m2;
+      if (KIND == K_GDN) d += ek[j] * eq[j];               // (scaled, so not to overflow or vanish without the norms)
+      yq[j] = byte_digits(eq[j]); yk[j] = TWO ? byte_digits(ek[j]) : 0u;
+    }
     if constexpr (AXV) {                    // every warp scales the vectors by its group's column scales, per stage
       *reinterpret_cast<float4*>(wq + lane * CW) = make_float4(eq[0], eq[1], eq[2], eq[3]);
       *reinterpret_cast<float4*>(wk + lane * CW) = make_float4(ek[0], ek[1], ek[2], ek[3]);
@@ -459,7 +472,7 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
       round_key(kr, mx);
     } else {
-      // the buffered keys' dot products with q and k: the key tile [M, 128] int8 is the A operand (rows = slots),
+      // the buffered keys' dot products with q and k, in the unit of the state's sums: the key tile [M, 128] int8 is the A operand (rows = slots),
       // the B fragments are those of the state pass (the 8-bit layout: the key tile holds bytes)
       __syncwarp();
       uint32_t bf8[8];
@@ -471,7 +484,7 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       SQB_STAMP(15);
       if (lane == 0) misc[2] = landed ? 0.f : 1.f;          // "a copy never arrived" flag
       const float ksl = ksv[lane];                          // scale of buffered key `lane`
-      const float iq1 = fq.i1, iq2 = fq.i2, ik1 = fk.i1, ik2 = fk.i2;
+      const int nlive = __float_as_int(misc[1]);            // (published before the named barrier)
       for (int sb = 0; sb < M; sb += 16) {
         int acc[4] = {MAGIC_I, MAGIC_I, MAGIC_I, MAGIC_I};
         int srow = sb + ((lane >> 3) & 1) * 8 + (lane & 7);       // slot whose row this lane addresses
@@ -488,8 +501,8 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
         float p[4] = {(__int_as_float(acc[0]) - 12582912.0f) * k0s, (__int_as_float(acc[1]) - 12582912.0f) * k0s,
                       (__int_as_float(acc[2]) - 12582912.0f) * k1s, (__int_as_float(acc[3]) - 12582912.0f) * k1s};
         float T = join_digits(p, t);          // t = 0: q, slot sb + i8; t = 1: q, slot sb + i8 + 8; t = 2, 3: k
-        T = t < 2 ? (T * iq1) * iq2 : (T * ik1) * ik2;
         const int slot = sb + i8 + (t & 1) * 8;
+        if (slot >= nlive) T = 0.f;                               // dead entries may hold anything
         if (slot < M) {
           if (t < 2) dqk[slot].x = T;
           else dqk[slot].y = T;
@@ -500,19 +513,20 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     // warp 3
     load_v();
     float qr[CW], kr[CW];
-    cvt4_raw(rq, dt_qk, qr);
-    cvt4_raw(rk, dt_qk, kr);
+    cvt4_raw<BIO>(rq, dt_qk, qr);
+    cvt4_raw<BIO>(rk, dt_qk, kr);
     if constexpr (!VDEC) {
-      // the key that goes into the buffer, rounded: its normalisation is redone here (the arithmetic of warp 0, so
-      // the same bits)
+      // the vectors' norms, and the key that goes into the buffer, rounded
       float s1 = 0.f;
-#pragma unroll
-      for (int j = 0; j < CW; j++) s1 += kr[j] * kr[j];
       if (KIND != K_M2) {
+        float s0 = 0.f;
+#pragma unroll
+        for (int j = 0; j < CW; j++) { s0 += qr[j] * qr[j]; s1 += kr[j] * kr[j]; }
+        s0 = warp_sum(s0);
         s1 = warp_sum(s1);
         const float nk = __fsqrt_rn(s1 + 1e-6f);
-#pragma unroll
-        for (int j = 0; j < CW; j++) kr[j] = __fdiv_rn(kr[j], nk);
+        if (lane == 0) { misc[9] = __fdiv_rn(A.scale, __fsqrt_rn(s0 + 1e-6f)); misc[10] = __fdiv_rn(1.0f, nk); }
+        div_norm(kr, nk);
       }
       float mx = 0.f;
 #pragma unroll
@@ -599,7 +613,6 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     for (int r = 0; r < 8; r++) bf[r] = Bfw[r * 32 + lane];
     acc_start<BITS, UPG>(bf, ci);
   }
-  const float kq = misc[0];
   const int n0 = __float_as_int(misc[1]);                       // live buffer entries of this slot
   const bool FOLD = CANFOLD && n0 == M - 1;                     // this token fills the buffer: fold after the read-out
   if (warp == KEY_WARP) {
@@ -619,9 +632,38 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       }
     }
   }
-  const float iq1 = misc[4], iq2 = misc[5], ik1 = misc[6], ik2 = misc[7];
-  const float2 dq01 = dqk[0];
+  // back to the vectors' own size and, for Gated DeltaNet, over the norm: powers of two (exact) and one factor per vector
+  const float iq1 = KIND == K_GDN ? misc[4] * misc[9] : misc[4], iq2 = misc[5];
+  const float ik1 = KIND == K_GDN ? misc[6] * misc[10] : misc[6], ik2 = misc[7];
+  const float kq = KIND == K_GDN ? (((misc[0] * iq1) * iq2) * ik1) * ik2 : misc[0];
   bool lost = false;
+  // What the buffered tokens add to the sums of this lane's row (head hi of the CTA, its buffered values ub, DV apart).  Decays
+  // per head: entries beyond the live ones weigh nothing and are finite, so they are taken without a branch each, and the sums
+  // are brought back to the vectors' size here; KDA's are in that size already.
+  auto buffer_terms = [&](const int8_t* ub, const float2* dc, float& tq, float& tk) {
+    auto term = [&](int i) {
+      const float2 du = dc[i], dd = dqk[i];
+      const float x = static_cast<float>(ub[i * DV]) * du.y;
+      tq = fmaf(x, du.x * dd.x, tq);
+      if (TWO) tk = fmaf(x, du.x * dd.y, tk);
+    };
+    if (!VDEC && MODE == 3 && TFMT) {                          // (a buffer of 8)
+      if (n0 > 0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) term(i);
+        if (n0 > 4) {
+#pragma unroll
+          for (int i = 4; i < 7; i++) term(i);
+        }
+      }
+    } else {
+      for (int i = 0; i < n0; i++) term(i);                    // live slots only; dead ones may hold garbage
+    }
+    if (!VDEC) {
+      tq = (tq * iq1) * iq2;
+      if (TWO) tk = (tk * ik1) * ik2;
+    }
+  };
 
   // rounds the u of this lane's row of stage sh and appends it; returns the dequantised rounded value
   auto append_row = [&](int sh) -> float {
@@ -646,8 +688,9 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
     return cc * usc;
   };
 
-  if (!FOLD && NSH == 2 && nst >= 2) {
-    // ---- a token that does not fold, two stages: both at once -----------------------------------------------------------
+  const bool both = !VDEC && NSH == 2 && nst >= 2 && (TFMT || !FOLD);      // (KDA has one stage; a fold in fp32 takes them one by one)
+  if (both) {
+    // ---- two stages at once -----------------------------------------------------------------------------------------
     // Both stages were requested in the CTA's first instructions; once both have landed, the two tile passes, the two
     // buffer terms and the two read-outs are independent chains in the same basic blocks, and the instruction scheduler
     // interleaves them (a warp issues in order: one chain alone leaves it waiting on every tensor-core and
@@ -676,21 +719,14 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       } else {
         tile_pass<BITS, UPG>(smem_u32(stA), reinterpret_cast<const unsigned short*>(stA + P.sc_off), bf, ci, warp, lane, tqA, tkA);
         tile_pass<BITS, UPG>(smem_u32(stB), reinterpret_cast<const unsigned short*>(stB + P.sc_off), bf, ci, warp, lane, tqB, tkB);
-        tqA = (tqA * iq1) * iq2; tqB = (tqB * iq1) * iq2;       // powers of two: exact
-        if (TWO) { tkA = (tkA * ik1) * ik2; tkB = (tkB * ik1) * ik2; }
+        if (VDEC) { tqA = (tqA * iq1) * iq2; tqB = (tqB * iq1) * iq2; tkA = (tkA * ik1) * ik2; tkB = (tkB * ik1) * ik2; }
       }
       if (!VDEC) { tqA = hdaA.w * tqA; tkA = hdaA.w * tkA; tqB = hdaB.w * tqB; tkB = hdaB.w * tkB; }
       const int8_t* ubA = reinterpret_cast<const int8_t*>(stA + P.ub_off) + hh * M * DV + rv;
       const int8_t* ubB = reinterpret_cast<const int8_t*>(stB + P.ub_off) + hh * M * DV + rv;
       const float2 *dcA = dcu + hiA * M, *dcB = dcu + hiB * M;
-      for (int i = 0; i < n0; i++) {                           // live slots only; dead ones may hold garbage
-        const float2 dd = i == 0 ? dq01 : dqk[i];
-        const float2 duA = dcA[i], duB = dcB[i];
-        const float xA = static_cast<float>(ubA[i * DV]) * duA.y, xB = static_cast<float>(ubB[i * DV]) * duB.y;
-        tqA = fmaf(xA, duA.x * dd.x, tqA);
-        tqB = fmaf(xB, duB.x * dd.x, tqB);
-        if (TWO) { tkA = fmaf(xA, duA.x * dd.y, tkA); tkB = fmaf(xB, duB.x * dd.y, tkB); }
-      }
+      buffer_terms(ubA, dcA, tqA, tkA);
+      buffer_terms(ubB, dcB, tqB, tkB);
       float uA, oA, uB, oB;
       if (KIND == K_GDN) {
         uA = hdaA.y * fmaf(-hdbA.x, tkA, vtA); oA = fmaf(kq, uA, hdbA.x * tqA);
@@ -713,9 +749,7 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       if (lane < 4 / WPH) { red[hiA * NW + warp % WPH + lane * WPH] = mA; red[hiB * NW + warp % WPH + lane * WPH] = mB; }
     }
   } else
-  for (int sh = 0; sh < NSH; sh++) {
-    const int s = sh % nst;
-    const uint32_t parity = (sh / nst) & 1;
+  for (int sh = 0, s = 0, parity = 0; sh < NSH; sh++) {
     const int hi = sh * HPS + hh, h = h0 + hi;
     uint8_t* st = smraw + P.stage0 + s * P.stage_bytes;
     const unsigned short* scs = reinterpret_cast<const unsigned short*>(st + P.sc_off);
@@ -738,18 +772,11 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
       if (TWO) tk = (tk * fk.i1) * fk.i2;
     } else {
       tile_pass<BITS, UPG>(smem_u32(st), scs, bf, ci, warp, lane, tq, tk);
-      tq = (tq * iq1) * iq2;                                  // powers of two: exact
-      if (TWO) tk = (tk * ik1) * ik2;
+      if (VDEC) { tq = (tq * iq1) * iq2; tk = (tk * ik1) * ik2; }
     }
     SQB_STAMP(6 + 3 * (sh & 1));
     if (!VDEC) { tq = alpha * tq; tk = alpha * tk; }
-    for (int i = 0; i < n0; i++) {                             // live slots only; dead ones may hold garbage
-      const float2 du = dcf[i];
-      const float2 dd = i == 0 ? dq01 : dqk[i];
-      const float ub = static_cast<float>(ubt[i * DV + rv]) * du.y;
-      tq = fmaf(ub, du.x * dd.x, tq);
-      if (TWO) tk = fmaf(ub, du.x * dd.y, tk);
-    }
+    buffer_terms(ubt + rv, dcf, tq, tk);
     float u, o;
     if (KIND == K_GDN) {
       u = beta * fmaf(-a, tk, vt);
@@ -889,12 +916,13 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
         }
       }
     }
+    if (++s == nst) { s = 0; parity ^= 1; }
   }
-  if (!FOLD) {
+  if (!FOLD || both) {
     // ---- append the values of all heads at slot n0, every lane its own rows ----
     if (__syncthreads_or(lost)) { bail(); return; }
     SQB_STAMP(11);
-    if (NSH == 2) {
+    if (!VDEC && NSH == 2) {
       // the two stages' rows of this lane at once: one address computation, packed arithmetic, the exact rounding of a
       // near-tie or of a subnormal scale out of line
       const int hiA = hh, hiB = HPS + hh;
@@ -918,12 +946,49 @@ __global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((B
         const int h = h0 + tid;
         const float4 r4 = *reinterpret_cast<const float4*>(red + tid * NW);
         UBSseq[h * M + n0] = f2h(fp16_scale(fmaxf(fmaxf(r4.x, r4.y), fmaxf(r4.z, r4.w)), 127.0f));
-        if (!VDEC) {
-          const float gnew = hd[tid * HD_W + 5];
-          GBseq[(long long)h * M + n0] = gnew;
-          GCseq[h] = gnew;
+        const float gnew = hd[tid * HD_W + 5];
+        GBseq[(long long)h * M + n0] = gnew;
+        GCseq[h] = FOLD ? 0.f : gnew;
+        NPseq[h] = FOLD ? 0 : n0 + 1;
+      }
+      if constexpr (CANFOLD && TFMT && !VDEC) {
+        if (FOLD) {
+          // ---- the fold on the tensor pipe (fold_mma.cuh), a stage after the other, both still in shared memory ----
+          float *ksf = fsm + P.ksf, *tab = fsm + P.tab;
+          uint32_t* KBf = reinterpret_cast<uint32_t*>(smraw + P.kbf);
+          us[hiA * DV + rv] = cc.x * ss.x;                      // this token's values as stored
+          us[hiB * DV + rv] = cc.y * ss.y;
+          mbar_wait(&bars[nst], 0, A.wait_ns);                  // the key tile has landed (warp 0 saw it before)
+          if (tid < 8) ksf[tid] = tid < 7 ? ksv[tid] : misc[8];
+          build_key_frags<BITS>(KBf, reinterpret_cast<const int8_t*>(kbt), reinterpret_cast<const int8_t*>(smraw + P.kcur), tid);
+          if (tid < 2 * HPS * 8) {                              // per head: decays and value scales of the slots
+            const int hq = tid >> 3, i = tid & 7;
+            const float gnew = hd[hq * HD_W + 5];
+            tab[hq * 20 + i] = i == 7 ? 1.0f : expf(gnew - fsm[P.gbs + tid]);
+            tab[hq * 20 + 8 + i] = dcu[tid].y;
+            if (i == 0) tab[hq * 20 + 16] = expf(gnew);
+          }
+          __syncthreads();
+#pragma unroll 1
+          for (int sh = 0; sh < 2; sh++) {
+            uint8_t* st = smraw + P.stage0 + sh * P.stage_bytes;
+            unsigned short* scs = reinterpret_cast<unsigned short*>(st + P.sc_off);
+            const int8_t* ub0 = reinterpret_cast<const int8_t*>(st + P.ub_off);
+            const float *u0 = us + sh * HPS * DV, *tb = tab + sh * HPS * 20;
+            if constexpr (AXV && BITS == 8) fold_stage_mma_v8<DV>(smem_u32(st), scs, ub0, u0, tb, ksf, KBf, warp, lane);
+            else if constexpr (AXV) fold_stage_mma_v4<DV>(smem_u32(st), scs, ub0, u0, tb, ksf, KBf, warp, lane);
+            else fold_stage_mma<BITS, UPG, DV>(smem_u32(st), scs, ub0, u0, tb, ksf, KBf, warp, lane);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+            if (warp == 0) {                                    // the stage goes back to the slot
+              const long long row0 = (long long)h0 * DV + sh * 128;
+              if (lane == 0) tile_s2g(&codes_map, static_cast<int>(row0), static_cast<int>(seq), st);
+              else if (lane == 1) bulk_s2g(SCseq + row0 * NG * 2, st + P.sc_off, 128 * NG * 2);
+              bulk_commit();
+            }
+          }
+          if (warp == 0) bulk_wait_read();                      // before leaving
         }
-        NPseq[h] = n0 + 1;
       }
     } else {
       for (int sh = 0; sh < NSH; sh++) append_row(sh);

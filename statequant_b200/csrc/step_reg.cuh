@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   rq.v = make_uint4(0u, 0u, 0u, 0u); rk.v = rq.v; rq.vec = false; rk.vec = false;
   const bool has_col = lane * CW < DK;                     // warps 0 and 3: four columns per lane
   if ((warp == 0 || warp == 3) && has_col) {
-    rq = ld4_raw(A.q + (long long)b * A.sq, dt_qk, (long long)hk * DK + lane * CW);
-    rk = ld4_raw(A.k + (long long)b * A.sk, dt_qk, (long long)hk * DK + lane * CW);
+    rq = ld4_raw<BIO>(A.q + (long long)b * A.sq, dt_qk, (long long)hk * DK + lane * CW);
+    rk = ld4_raw<BIO>(A.k + (long long)b * A.sk, dt_qk, (long long)hk * DK + lane * CW);
   }
   long long seq = b;
   if (A.idx != nullptr) {
@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     // q and k as they come, scaled by powers of two (integer states: 30-bit fixed point, mma_pass.cuh); what their norms make
     // of the results, warp 3 finds out meanwhile and every row applies at the end
     float qr[CW], kr[CW];
-    cvt4_raw(rq, dt_qk, qr);
-    cvt4_raw(rk, dt_qk, kr);
+    cvt4_raw<BIO>(rq, dt_qk, qr);
+    cvt4_raw<BIO>(rk, dt_qk, kr);
     float d = 0.f, mq = 0.f, mk = 0.f;
 #pragma unroll
     for (int j = 0; j < CW; j++) { mq = fmaxf(mq, fabsf(qr[j])); mk = fmaxf(mk, fabsf(kr[j])); }
@@ -290,10 +290,10 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   } else if (warp == 3) {
     // the norms, and the key as it goes into the buffer
     float kr[CW];
-    cvt4_raw(rk, dt_qk, kr);
+    cvt4_raw<BIO>(rk, dt_qk, kr);
     if (KIND != K_M2) {
       float qr[CW], s0 = 0.f, s1 = 0.f;
-      cvt4_raw(rq, dt_qk, qr);
+      cvt4_raw<BIO>(rq, dt_qk, qr);
 #pragma unroll
       for (int j = 0; j < CW; j++) { s0 += qr[j] * qr[j]; s1 += kr[j] * kr[j]; }
       s0 = warp_sum(s0);
@@ -534,8 +534,7 @@ int launch_reg_one(const StepArgs& a, cudaStream_t stream) {
   StepArgs b = a;
   b.gqa_full = a.HV / a.HK;
   const dim3 grid(static_cast<unsigned>(a.rows), static_cast<unsigned>(a.HV / HPS));
-  // bf16 activations and output take the kernel with those element types compiled in
-  const bool bio = a.dt_qk == DT_BF16 && a.dt_v == DT_BF16 && a.dt_out == DT_BF16;
+  const bool bio = bf16_io(a);              // takes the kernel with those element types compiled in
   auto kern = bio ? step_reg_kernel<KIND, BITS, DK, DV, HPS, true> : step_reg_kernel<KIND, BITS, DK, DV, HPS, false>;
   static Residency residency[2];
   const bool early = enters_early(static_cast<long long>(grid.x) * grid.y, residency[bio].ctas(kern, HPS * DV, 0), false);
