@@ -7,14 +7,14 @@
 
 namespace sqb {
 
-// Shapes the tensor-core kernels take: 4 / 8-bit codes scaled along k in groups of 32, 64 or 128, d_k 128, d_v 64 or
-// 128 (whole stages of 128 rows per key head), int8 buffer, q / k per key head, every per-head chunk and table
+// Shapes the tensor-core kernels take: 4 / 8-bit codes scaled along k in groups of 32, 64 or 128, d_k 128, d_v 128 or (Mamba2)
+// 64 (whole stages of 128 rows per key head), int8 buffer, q / k per key head, every per-head chunk and table
 // stride a multiple of 16 bytes.
 // Scaled along v: 4- or 8-bit codes in groups of 32 rows, Gated DeltaNet, buffer length 8 (the fold inside the step kernel
 // is the tensor-pipe one).
 inline bool mma_shape_ok(const StepArgs& a, int bits, bool axk, bool kda, int kind = K_GDN) {
   if ((bits != 4 && bits != 8) || a.DK != 128 || !a.qbuf) return false;
-  if (a.DV != 64 && a.DV != 128) return false;
+  if (a.DV != 128 && !(a.DV == 64 && kind == K_M2)) return false;       // (heads of 64 rows: instances for Mamba2 only)
   if (!axk) {
     if (a.group != 32 || kind != K_GDN || a.M != 8 || a.DV != 128) return false;
   } else if (a.group != 32 && a.group != 64 && a.group != 128) return false;

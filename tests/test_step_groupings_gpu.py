@@ -31,6 +31,19 @@ def test_tensor_core_step_over_head_groupings(fmt, hv, hk):
     assert st['buf'] <= max(1, 1e-4 * st['nbuf']) and st['codes'] <= max(1, 1e-4 * st['ncodes']) and st['scal'] <= max(1, 1e-4 * st['ncodes']), st
 
 
+@pytest.mark.parametrize('fmt', [(4, 'k', 64), (8, 'k', 32)])
+def test_heads_of_64_rows_where_the_tensor_core_step_is_asked_for(fmt):
+    """Gated DeltaNet heads of 64 rows run on the next kernel that takes them (grids beyond one wave come here by themselves)."""
+    from statequant_b200 import _cabi
+    _cabi.set_option('kernel_path', 4)
+    try:
+        st = _oracle_lockstep(dict(kind='gdn', fmt=fmt, B=2, hv=4, hk=2, dk=128, dv=64, m=8, bb=8, seed=102), T=19, act_dtype=torch.float32)
+    finally:
+        _cabi.set_option('kernel_path', 0)
+    assert st['worst'] < 2e-5, st
+    assert st['buf'] <= max(1, 1e-4 * st['nbuf']) and st['codes'] <= max(1, 1e-4 * st['ncodes']) and st['scal'] <= max(1, 1e-4 * st['ncodes']), st
+
+
 @pytest.mark.parametrize('fmt,dk,dv,path', [((8, 'k', 32), 128, 128, 4), ((8, 'k', 32), 128, 128, 5), ((4, 'v', 32), 128, 128, 4),
                                             ((4, 'k', 64), 96, 192, 5), ('bf16', 128, 128, 5)])
 @pytest.mark.parametrize('skew', [1, 2, 3])
