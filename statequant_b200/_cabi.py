@@ -125,7 +125,9 @@ def check(rc, what):
 
 
 def current_stream(device):
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """Handle of the calling thread's current stream on a tensor's device (without a Stream object around it: a step call is
+    bound by the host where the batch is small)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def launch_count():
