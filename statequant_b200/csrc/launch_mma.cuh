@@ -60,20 +60,34 @@ inline bool mma_plan(const StepArgs& a, int bits, int mode, SmemM& plan, int& ns
   return plan.total <= 220 * 1024;
 }
 
-template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV, bool BIO>
+template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV, bool BIO, int RES>
 int launch_mma_one_io(const StepArgs& a, cudaStream_t stream);
+
+// Seven CTAs an SM instead of five cost a 4-bit kernel a few spilled registers (72 instead of 96) and pay where the launch is long enough.
+// us per layer-step at five / seven, slots on one token and each on its own.  KDA, 640 CTAs 7.6 / 8.1 and 12.4 / 13.2, 1024 mixed 16.3 / 14.5,
+// 1536 same 16.4 / 15.8, 3072 mixed 35.3 / 34.5, 6400 54.9 / 52.6 and 67.7 / 63.7: beyond one wave of five.  Gated DeltaNet, 768 CTAs 10.6 / 9.8 and
+// 15.8 / 16.4, 1536 17.5 / 16.9 and 23.5 / 24.3, 3072 mixed 38.1 / 38.3, 4096 38.8 / 37.2 and 48.1 / 47.3, 65536 mixed 642 / 608: beyond five waves, where
+// both gain.  Mamba2, states scaled along v and 8-bit codes (shared memory holds five) lose: 45.2 / 46.2, 45.1 / 46.7, 37.5 / 38.0.
+template <int KIND, int BITS, int UPG, int MODE, bool AXV>
+constexpr bool mma_has_seven() { return MODE == 3 && BITS == 4 && UPG == 2 && !AXV && KIND != K_M2; }
+inline bool mma_takes_seven(int kind, long long ctas) { return ctas > (kind == K_KDA ? 1 : 5) * 5 * 148; }
 
 // bf16 activations and output (bf16_io) take the kernel with those element types compiled in
 template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV = false>
 int launch_mma_one(const StepArgs& a, cudaStream_t stream) {
-  if (bf16_io(a))
-    return launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, true>(a, stream);
-  return launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, false>(a, stream);
+  constexpr int RES = mma_residency(BITS, UPG, MODE, AXV);
+  if constexpr (mma_has_seven<KIND, BITS, UPG, MODE, AXV>()) {
+    if (mma_takes_seven(KIND, static_cast<long long>(a.rows) * (a.HV / mma_hpc(a))))
+      return bf16_io(a) ? launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, true, 7>(a, stream)
+                        : launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, false, 7>(a, stream);
+  }
+  return bf16_io(a) ? launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, true, RES>(a, stream)
+                    : launch_mma_one_io<KIND, BITS, UPG, DV, MODE, AXV, false, RES>(a, stream);
 }
 
-template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV, bool BIO>
+template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV, bool BIO, int RES>
 int launch_mma_one_io(const StepArgs& a, cudaStream_t stream) {
-  auto kern = step_mma_kernel<KIND, BITS, UPG, DV, MODE, AXV, BIO>;
+  auto kern = step_mma_kernel<KIND, BITS, UPG, DV, MODE, AXV, BIO, RES>;
   SmemM plan;
   int nst;
   if (!mma_plan<KIND>(a, BITS, MODE, plan, nst)) return 1;

@@ -101,22 +101,12 @@ __host__ __device__ inline SmemM smemm_plan(int kind, int bits, int upg, int DV,
   return s;
 }
 
-#ifndef SQB_MMA_MINB8
-#define SQB_MMA_MINB8 5
-#endif
-#ifndef SQB_MMA_MINB4
-#define SQB_MMA_MINB4 6
-#endif
-
-#ifndef SQB_MMA_MINB_FOLD
-#define SQB_MMA_MINB_FOLD 4
-#endif
-#ifndef SQB_MMA_MINB_TFOLD
-#define SQB_MMA_MINB_TFOLD 5
-#endif
-#ifndef SQB_MMA_MINB_AXV
-#define SQB_MMA_MINB_AXV 5
-#endif
+// CTAs of a step kernel that an SM's registers are to hold: 96 registers for five, 80 for six, 72 for seven (launch_mma.cuh has what
+// launches take seven).
+constexpr int mma_residency(int bits, int upg, int mode, bool axv) {
+  if (mode != 3) return bits == 4 ? 6 : 5;
+  return axv || (bits == 8 && upg == 1) || (bits == 4 && upg == 2) ? 5 : 4;
+}
 
 // Cold paths kept out of line (they are never taken in a healthy run, and inlined at every use they were an eighth of
 // the kernel's code): the zero fill of a CTA's output rows, and the exit of a CTA whose copy never completed.
@@ -135,9 +125,8 @@ static __device__ __noinline__ void mma_bail(uint8_t* orow, int dt, int n, uint6
 
 // BIO: q / k / v and the output are bf16, q and k on 8-byte boundaries (what a serving engine passes): the element types of the activation loads and
 // stores are then compile-time constants instead of three-way run-time dispatches at every access.
-template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV = false, bool BIO = false>
-__global__ void __launch_bounds__(NT, MODE == 3 ? (AXV ? SQB_MMA_MINB_AXV : (((BITS == 8 && UPG == 1) || (BITS == 4 && UPG == 2)) ? SQB_MMA_MINB_TFOLD : SQB_MMA_MINB_FOLD))
-                                               : (BITS == 4 ? SQB_MMA_MINB4 : SQB_MMA_MINB8))
+template <int KIND, int BITS, int UPG, int DV, int MODE, bool AXV, bool BIO, int RES>
+__global__ void __launch_bounds__(NT, RES)
     step_mma_kernel(const __grid_constant__ StepArgs A, const __grid_constant__ TileMap codes_map, const __grid_constant__ SmemM P,
                     const int nst) {
   dependency_wait();
