@@ -34,8 +34,9 @@ namespace sqb {
 
 // Threads per SM: bf16 holds 64 words of state per thread (128 registers); integer states of d_k 128 come here in grids of up
 // to four CTAs per SM, and need the registers more than the residency; those of d_k 96 in grids of any size (80 registers:
-// 852 us a pass against 955 us with 112).  What the caps cost (ptxas): 96-wide instances spill 16 .. 56 bytes (28 .. 68 loaded), bf16
-// ones 12 .. 24 (16 .. 40), 8-bit ones of d_k 128 up to 16, 4-bit ones of d_k 128 nothing.
+// 852 us a pass against 955 us with 112).  What the caps cost (ptxas): 96-wide instances spill 4 .. 56 bytes (4 .. 64
+// loaded), bf16 ones up to 20 (36), integer ones of d_k 128 nothing.  (No lambda in this kernel captures by reference what another part
+// of it keeps in registers: one that did cost the bf16 instances 20 bytes of spills and 9 % of their time.)
 constexpr int reg_min_ctas(int bits, int dk, int threads) { return (bits == 16 || dk == 128 ? 512 : 768) / threads; }
 
 // N words of a lane's slice of a unit: 4 (bf16), 2 (int8) or 1 (int4)
@@ -116,6 +117,34 @@ __device__ __forceinline__ void gates_finish(const StepArgs& A, const GateRaw& w
 // the sum of a hi + mid + lo triple whose lower parts may be 0 * inf: a hi part that is not finite stands alone
 __device__ __forceinline__ float add_parts(float hi, float lo) { return fabsf(hi) <= 3.402823466e38f ? hi + lo : hi; }
 
+// The fold of NH units, from unit h0 on, of a block's rows g and g + 8 (words w0, w1; scales sc by group): fresh codes to Sx (the
+// lane's place in row g of the block) and scales to SCx.
+template <int BITS, int UPG, int NH, int NG, int ROWB>
+__device__ __forceinline__ void reg_fold_chunk(const uint32_t* w0, const uint32_t* w1, const float (&sc)[2][UPG == 1 ? NH : 1],
+                                               const uint32_t (&A1)[2], const uint32_t (&A2)[2], const uint32_t (&A3)[2],
+                                               const uint32_t* KBf, int h0, int lane, float2 al2, uint8_t* Sx, unsigned short* SCx) {
+  constexpr int NS = UPG == 1 ? NH : 1, WPU = BITS / 4;
+  const int t = lane & 3;
+  uint32_t m[NH][4], o[NH][4];
+  float acc[NH][4][4];
+#pragma unroll
+  for (int n = 0; n < NH; n++) {
+#pragma unroll
+    for (int p = 0; p < WPU; p++) { m[n][2 * p] = w0[n * WPU + p]; m[n][2 * p + 1] = w1[n * WPU + p]; }
+  }
+  fold_acc<BITS, UPG, NH, false>(m, sc, A1, A2, A3, KBf, h0, lane, al2, nullptr, acc);
+  const float s_own = fold_round<BITS, UPG, NH>(acc, lane, o);
+  if (NS == 2 || t < 2) SCx[8 * (t & 1) * NG + h0 / UPG + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);
+#pragma unroll
+  for (int n = 0; n < NH; n++) {
+    uint32_t a[WPU], c[WPU];
+#pragma unroll
+    for (int p = 0; p < WPU; p++) { a[p] = o[n][2 * p]; c[p] = o[n][2 * p + 1]; }
+    st_words<WPU>(Sx + 4 * BITS * (h0 + n), a);
+    st_words<WPU>(Sx + 8 * ROWB + 4 * BITS * (h0 + n), c);
+  }
+}
+
 template <int KIND, int BITS, int DK, int DV, int HPS, bool BIO>
 __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) step_reg_kernel(const __grid_constant__ StepArgs A) {
   dependency_wait();
@@ -142,13 +171,21 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   const int b = blockIdx.x, h0 = blockIdx.y * HPS, hk = h0 / A.gqa_full;
   const bool first = h0 == hk * A.gqa_full;                // the CTA that appends the key head's key
   const int osz = dt_size(dt_out);
+  // Roles: warp 0 makes the fragments of q and k; in a CTA of six warps of q only, and warp 4 those of k (everybody waits for the
+  // longest of them: 96 x 192, int4 k/64, 64 rows of 30 heads 24.9 -> 20.5 us; in a CTA of four warps another warp's work would have to
+  // move for it, and a small grid loses 4 %); warp 1 the gates, warp 2 the decays, warp 3 the norms and the key.
+  constexpr int NVEC = NT > 128 ? 1 : 2;
+  const bool makes = warp == 0 || (NVEC == 1 && warp == 4);
+  const int vec0 = warp == 0 ? 0 : 1;
   // q and k leave before the slot index is known
-  Raw4 rq, rk;
-  rq.v = make_uint4(0u, 0u, 0u, 0u); rk.v = rq.v; rq.vec = false; rk.vec = false;
-  const bool has_col = lane * CW < DK;                     // warps 0 and 3: four columns per lane
-  if ((warp == 0 || warp == 3) && has_col) {
-    rq = ld4_raw<BIO>(A.q + (long long)b * A.sq, dt_qk, (long long)hk * DK + lane * CW);
-    rk = ld4_raw<BIO>(A.k + (long long)b * A.sk, dt_qk, (long long)hk * DK + lane * CW);
+  Raw4 rqk[2];
+#pragma unroll
+  for (int v = 0; v < 2; v++) { rqk[v].v = make_uint4(0u, 0u, 0u, 0u); rqk[v].vec = false; }
+  const bool has_col = lane * CW < DK;                     // four columns per lane
+  if (has_col && (makes || warp == 3)) {
+    const uint8_t *q = A.q + (long long)b * A.sq, *k = A.k + (long long)b * A.sk;
+    rqk[0] = ld4_raw<BIO>(NVEC == 1 && warp == 4 ? k : q, dt_qk, (long long)hk * DK + lane * CW);
+    if (NVEC == 2 || warp == 3) rqk[1] = ld4_raw<BIO>(k, dt_qk, (long long)hk * DK + lane * CW);
   }
   long long seq = b;
   if (A.idx != nullptr) {
@@ -168,13 +205,13 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   float* GCseq = reinterpret_cast<float*>(A.GCUR + seq * A.sGC);
 
   // ---- every fetch: a role's small ones first (they head the serial chains), then the state, then the buffered values --
-  uint2 kw[NU];                                            // warp 0: slot g of the key tile, its 8 columns of every unit
+  uint2 kw[NU];                                            // fragments' warps: slot g of the key tile, its 8 columns of every unit
   float ksl = 0.f;
   GateRaw gr;
   int nraw = 0;
   float gb0 = 0.f, gc0 = 0.f;
   unsigned short us0 = 0;
-  if (warp == 0) {
+  if (makes) {
 #pragma unroll
     for (int u = 0; u < NU; u++) kw[u] = *reinterpret_cast<const uint2*>(KBh + g * DK + 32 * u + 8 * t);
     ksl = h2f(KBSh[g]);
@@ -215,45 +252,51 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   // ---- prologue, by role ----------------------------------------------------------------------------------------
   uint32_t kword = 0;                                      // warp 3: the key as it goes into the buffer
   float kscale = 0.f;
-  if (warp == 0) {
+  if (makes) {
     // q and k as they come, scaled by powers of two (integer states: 30-bit fixed point, mma_pass.cuh); what their norms make
-    // of the results, warp 3 finds out meanwhile and every row applies at the end
-    float qr[CW], kr[CW];
-    cvt4_raw<BIO>(rq, dt_qk, qr);
-    cvt4_raw<BIO>(rk, dt_qk, kr);
-    float d = 0.f, mq = 0.f, mk = 0.f;
+    // of the results, warp 3 finds out meanwhile and every row applies at the end.  (Mamba2 reads the state against q only.)
+    float x[NVEC][CW], mx[NVEC], d = 0.f;
+    FxScale fx[NVEC];
 #pragma unroll
-    for (int j = 0; j < CW; j++) { mq = fmaxf(mq, fabsf(qr[j])); mk = fmaxf(mk, fabsf(kr[j])); }
-    mq = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mq)));
-    mk = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mk)));
-    const FxScale fq = fx_scale<TOP>(mq), fk = fx_scale<TOP>(mk);
+    for (int v = 0; v < NVEC; v++) {
+      cvt4_raw<BIO>(rqk[v], dt_qk, x[v]);
+      mx[v] = 0.f;
+#pragma unroll
+      for (int j = 0; j < CW; j++) mx[v] = fmaxf(mx[v], fabsf(x[v][j]));
+    }
+#pragma unroll
+    for (int v = 0; v < NVEC; v++) {
+      mx[v] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx[v])));
+      fx[v] = fx_scale<TOP>(mx[v]);
+    }
 #pragma unroll
     for (int j = 0; j < CW; j++) {
-      if (KIND == K_M2) d += kr[j] * qr[j];                // C . B as it is
-      qr[j] = (qr[j] * fq.m1) * fq.m2;
-      kr[j] = (kr[j] * fk.m1) * fk.m2;
-      if (KIND != K_M2) d += kr[j] * qr[j];                // (the vectors' norms still missing, so not to overflow or vanish)
+      if (NVEC == 2 && KIND == K_M2) d += x[NVEC - 1][j] * x[0][j];        // C . B as it is
+#pragma unroll
+      for (int v = 0; v < NVEC; v++) x[v][j] = (x[v][j] * fx[v].m1) * fx[v].m2;
+      if (NVEC == 2 && KIND != K_M2) d += x[NVEC - 1][j] * x[0][j];        // (the vectors' norms still missing, so not to overflow or vanish)
     }
     // bf16: the state pass's fragments: lane l's columns 4 l .. 4 l + 3 are step l / 8 * 2 + l % 2, thread (l % 8) / 2
     if constexpr (!QUANT) {
-      uint2* bw = Bf + (2 * (lane >> 3) + (lane & 1)) * 32 + ((lane & 7) >> 1);
 #pragma unroll
-      for (int vec = 0; vec < 2; vec++) {
+      for (int v = 0; v < NVEC; v++) {
+        uint2* bw = Bf + (2 * (lane >> 3) + (lane & 1)) * 32 + ((lane & 7) >> 1) + 16 * (vec0 + v);
+        const bool on = TWO || vec0 + v == 0;
         float p[3][CW];
 #pragma unroll
-        for (int j = 0; j < CW; j++) split3(vec ? kr[j] : qr[j], p[0][j], p[1][j], p[2][j]);
+        for (int j = 0; j < CW; j++) split3(on ? x[v][j] : 0.f, p[0][j], p[1][j], p[2][j]);
 #pragma unroll
-        for (int s = 0; s < 4; s++)
-          bw[(4 * vec + s) * 4] = s == 3 || (vec && !TWO) ? make_uint2(0u, 0u) : make_uint2(bf2(p[s < 3 ? s : 0][0], p[s < 3 ? s : 0][1]),
-                                                                                       bf2(p[s < 3 ? s : 0][2], p[s < 3 ? s : 0][3]));
+        for (int s = 0; s < 3; s++) bw[s * 4] = make_uint2(bf2(p[s][0], p[s][1]), bf2(p[s][2], p[s][3]));
+        bw[12] = make_uint2(0u, 0u);
       }
     }
-    // the buffered keys against q and k: integer digits (mma_pass.cuh), the key codes straight from the loads
+    // the buffered keys against them: integer digits (mma_pass.cuh), the key codes straight from the loads
 #pragma unroll
-    for (int vec = 0; vec < 2; vec++) {
+    for (int v = 0; v < NVEC; v++) {
+      const int vec = vec0 + v;
       uint32_t y[CW];
 #pragma unroll
-      for (int j = 0; j < CW; j++) y[j] = vec == 0 ? byte_digits(qr[j] * UPF) : (TWO ? byte_digits(kr[j] * UPF) : 0u);
+      for (int j = 0; j < CW; j++) y[j] = TWO || vec == 0 ? byte_digits(x[v][j] * UPF) : 0u;
       const uint32_t t0 = __byte_perm(y[0], y[1], 0x5140), t1 = __byte_perm(y[2], y[3], 0x5140);
       const uint32_t t2 = __byte_perm(y[0], y[1], 0x7362), t3 = __byte_perm(y[2], y[3], 0x7362);
       const uint32_t W[4] = {__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410),
@@ -262,12 +305,20 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
       for (int s = 0; s < 4; s++) Bf8[(2 * (lane >> 3) + (lane & 1)) * 32 + (vec * 4 + 3 - s) * 4 + ((lane & 7) >> 1)] = W[s];
       if constexpr (BITS == 4) put_b_words<4>(Bf4, lane, vec, y[0], y[1], y[2], y[3]);
     }
-    d = warp_sum(d);
-    if (lane == 0) { misc[0] = d; misc[4] = fq.i1; misc[5] = fq.i2; misc[6] = fk.i1; misc[7] = fk.i2; }
+    if (NVEC == 2) d = warp_sum(d);
+    if (lane == 0) {
+      if (NVEC == 2) misc[0] = d;
 #pragma unroll
-    for (int u = 0; u < NU; u++) *reinterpret_cast<uint2*>(kbt + g * DK + 32 * u + 8 * t) = kw[u];
+      for (int v = 0; v < NVEC; v++) { misc[4 + 2 * (vec0 + v)] = fx[v].i1; misc[5 + 2 * (vec0 + v)] = fx[v].i2; }
+    }
+    if (vec0 == 0) {
+#pragma unroll
+      for (int u = 0; u < NU; u++) *reinterpret_cast<uint2*>(kbt + g * DK + 32 * u + 8 * t) = kw[u];
+      if (t == 0) ksf[g] = ksl;
+    }
     __syncwarp();
-    int acc[4] = {MAGIC_I, MAGIC_I, 0, 0};                 // fragment rows 8 .. 15 are empty
+    // (fragment rows 8 .. 15 are empty; one vector a warp: the other's columns may not be written yet, and are not looked at)
+    int acc[4] = {MAGIC_I, MAGIC_I, 0, 0};
 #pragma unroll
     for (int u = 0; u < NU; u++)
       mma_i8<false>(acc, kw[u].x, 0u, kw[u].y, 0u, Bf8[(2 * u) * 32 + lane], Bf8[(2 * u + 1) * 32 + lane]);
@@ -275,8 +326,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     float T = fmaf((__int_as_float(acc[0]) - 12582912.0f) * ksl, wa, ((__int_as_float(acc[1]) - 12582912.0f) * ksl) * wb);
     T += __shfl_xor_sync(0xffffffffu, T, 1);
     T *= 1.0f / UPF;                                       // (in the unit of the state's sums)
-    if (t == 0) { dqk[g].x = T; ksf[g] = ksl; }
-    if (t == 2) dqk[g].y = T;
+    if (!(t & 1) && (NVEC == 2 || (t >> 1) == vec0)) reinterpret_cast<float*>(dqk + g)[t >> 1] = T;
   } else if (warp == 1) {
     if (lane < HPS) gates_finish<KIND>(A, gr, hd + lane * HD_W);
   } else if (warp == 2) {
@@ -288,28 +338,37 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
       gbs[lane] = gb0;
     }
   } else if (warp == 3) {
-    // the norms, and the key as it goes into the buffer
+    // the norms, and the key as it goes into the buffer (one vector a warp: k . q as well)
+    static_assert(NVEC == 2 || KIND != K_M2, "C . B is summed by the warp that has both");
     float kr[CW];
-    cvt4_raw<BIO>(rk, dt_qk, kr);
+    cvt4_raw<BIO>(rqk[1], dt_qk, kr);
     if (KIND != K_M2) {
       float qr[CW], s0 = 0.f, s1 = 0.f;
-      cvt4_raw<BIO>(rq, dt_qk, qr);
+      cvt4_raw<BIO>(rqk[0], dt_qk, qr);
 #pragma unroll
       for (int j = 0; j < CW; j++) { s0 += qr[j] * qr[j]; s1 += kr[j] * kr[j]; }
       s0 = warp_sum(s0);
       s1 = warp_sum(s1);
-      const float nk = __fsqrt_rn(s1 + 1e-6f);
-      if (lane == 0) { misc[8] = __fdiv_rn(A.scale, __fsqrt_rn(s0 + 1e-6f)); misc[9] = __fdiv_rn(1.0f, nk); }
+      const float nk = __fsqrt_rn(s1 + 1e-6f), rn = __fdiv_rn(A.scale, __fsqrt_rn(s0 + 1e-6f));
+      if (lane == 0) { misc[8] = rn; misc[9] = __fdiv_rn(1.0f, nk); }
+      div_norm(kr, nk);
+      if constexpr (NVEC == 1) {
+        float d = 0.f;
 #pragma unroll
-      for (int j = 0; j < CW; j++) kr[j] = __fdiv_rn(kr[j], nk);
+        for (int j = 0; j < CW; j++) d += kr[j] * (qr[j] * rn);
+        d = warp_sum(d);
+        if (lane == 0) misc[0] = d;
+      }
     }
     float mx = 0.f;
 #pragma unroll
     for (int j = 0; j < CW; j++) mx = fmaxf(mx, fabsf(kr[j]));
     mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
     kscale = fp16_scale(mx, 127.0f);
+    float cc[CW];
+    round4(kr, kscale, cc);
 #pragma unroll
-    for (int j = 0; j < CW; j++) kword |= (static_cast<uint32_t>(static_cast<int>(rq_exact(kr[j], kscale, 127.0f))) & 0xFFu) << (8 * j);
+    for (int j = 0; j < CW; j++) kword |= (static_cast<uint32_t>(static_cast<int>(cc[j])) & 0xFFu) << (8 * j);
     if (has_col) *reinterpret_cast<uint32_t*>(kcur + lane * 4) = kword;
     if (lane == 0) misc[2] = kscale;
   }
@@ -318,7 +377,7 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
   // first power, so that no step between lies beyond the sum and the result: states near the largest float)
   const float iq1 = KIND == K_M2 ? misc[4] : misc[4] * misc[8], iq2 = misc[5];
   const float ik1 = KIND == K_M2 ? misc[6] : misc[6] * misc[9], ik2 = misc[7];
-  const float kq = KIND == K_M2 ? misc[0] : (((misc[0] * iq1) * iq2) * ik1) * ik2;
+  const float kq = KIND == K_M2 || NVEC == 1 ? misc[0] : (((misc[0] * iq1) * iq2) * ik1) * ik2;
   const int n0 = __float_as_int(misc[1]);                  // live buffer entries of this slot
   const bool full = n0 == M - 1;                           // this token fills the buffer: fold after the read-out
   if (warp == 3 && first) {
@@ -471,59 +530,67 @@ __global__ void __launch_bounds__(HPS * DV, reg_min_ctas(BITS, DK, HPS * DV)) st
     }
     __syncwarp();
     const float2 al2 = make_float2(tb[16], tb[16]);
+    if constexpr (!QUANT) {
 #pragma unroll
-    for (int x = 0; x < 2; x++) {
-      uint32_t A1[2], A2[2], A3[2];
+      for (int x = 0; x < 2; x++) {
+        uint32_t A1[2], A2[2], A3[2];
 #pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const uint32_t* l = Lp + (warp * 32 + 16 * x + 8 * r + g) * 12 + t;
-        A1[r] = l[0]; A2[r] = l[4]; A3[r] = l[8];
-      }
-      if constexpr (!QUANT) {
+        for (int r = 0; r < 2; r++) {
+          const uint32_t* l = Lp + (warp * 32 + 16 * x + 8 * r + g) * 12 + t;
+          A1[r] = l[0]; A2[r] = l[4]; A3[r] = l[8];
+        }
 #pragma unroll
         for (int un = 0; un < NU; un++) {
           const uint4 kf = *reinterpret_cast<const uint4*>(KBf + (un * 32 + lane) * 4);
           const uint32_t kb[4] = {kf.x, kf.y, kf.z, kf.w};
+          uint32_t a[4], c[4];
 #pragma unroll
           for (int p = 0; p < 4; p++) {                    // the two rows' words of one column pair
-            uint32_t &wa = sw[x][0][un * WPU + p], &wc = sw[x][1][un * WPU + p];
+            const uint32_t wa = sw[x][0][un * WPU + p], wc = sw[x][1][un * WPU + p];
             const float2 fa = __fmul2_rn(make_float2(__uint_as_float(wa << 16), __uint_as_float(wa & 0xFFFF0000u)), al2);
             const float2 fc = __fmul2_rn(make_float2(__uint_as_float(wc << 16), __uint_as_float(wc & 0xFFFF0000u)), al2);
             float acc[4] = {fa.x, fa.y, fc.x, fc.y};
             mma_bf16(acc, A1[0], A1[1], A2[0], A2[1], kb[p], kb[p]);
             mma_bf16_k8(acc, A3[0], A3[1], kb[p]);
-            wa = bf2(acc[0], acc[1]);
-            wc = bf2(acc[2], acc[3]);
+            a[p] = bf2(acc[0], acc[1]);
+            c[p] = bf2(acc[2], acc[3]);
           }
+          st_words<WPU>(Srow + 16 * x * ROWB + 4 * BITS * un, a);
+          st_words<WPU>(Srow + (16 * x + 8) * ROWB + 4 * BITS * un, c);
         }
-      } else {
-        auto halves = [&](auto nh, auto hc) {              // NH units from unit H0 on
-          constexpr int NH = decltype(nh)::value, H0 = decltype(hc)::value, NS = UPG == 1 ? NH : 1, G0 = H0 / UPG;
-          uint32_t m[NH][4], o[NH][4];
-          float sc[2][NS], acc[NH][4][4];
-#pragma unroll
-          for (int n = 0; n < NH; n++) {
-#pragma unroll
-            for (int p = 0; p < WPU; p++) { m[n][2 * p] = sw[x][0][(H0 + n) * WPU + p]; m[n][2 * p + 1] = sw[x][1][(H0 + n) * WPU + p]; }
-          }
-#pragma unroll
-          for (int i = 0; i < NS; i++) { sc[0][i] = scale_of(scr[x][0], G0 + i); sc[1][i] = scale_of(scr[x][1], G0 + i); }
-          fold_acc<BITS, UPG, NH, false>(m, sc, A1, A2, A3, KBf, H0, lane, al2, nullptr, acc);
-          const float s_own = fold_round<BITS, UPG, NH>(acc, lane, o);
-          if (NS == 2 || t < 2) SCrow[(16 * x + 8 * (t & 1)) * NG + G0 + (NS == 2 ? t >> 1 : 0)] = f2h(s_own);
-#pragma unroll
-          for (int n = 0; n < NH; n++) {
-#pragma unroll
-            for (int p = 0; p < WPU; p++) { sw[x][0][(H0 + n) * WPU + p] = o[n][2 * p]; sw[x][1][(H0 + n) * WPU + p] = o[n][2 * p + 1]; }
-          }
-        };
-        halves(IntC<2>(), IntC<0>());
-        halves(IntC<NU - 2>(), IntC<2>());
       }
+    } else {
+      // A loop over the blocks that moves the state's registers up behind it: unrolled, the fold was half of the kernel's code, and a
+      // token that folds now and then waits for instructions (1 row of 32 heads, int4 k/64: 6.2 -> 5.6 us).  A block's two halves stay
+      // side by side: each on its own in the loop, 37 rows of 8 heads with a slot in eight folding take 7.6 us a layer instead of 7.3.
+#pragma unroll 1
+      for (int x = 0; x < 2; x++) {
+        uint32_t A1[2], A2[2], A3[2];
 #pragma unroll
-      for (int r = 0; r < 2; r++) {
+        for (int r = 0; r < 2; r++) {
+          const uint32_t* l = Lp + (warp * 32 + 16 * x + 8 * r + g) * 12 + t;
+          A1[r] = l[0]; A2[r] = l[4]; A3[r] = l[8];
+        }
+        constexpr int NH2 = NU - 2;
+        float s0[2][UPG == 1 ? 2 : 1], s1[2][UPG == 1 ? NH2 : 1];
 #pragma unroll
-        for (int un = 0; un < NU; un++) st_words<WPU>(Srow + (16 * x + 8 * r) * ROWB + 4 * BITS * un, &sw[x][r][un * WPU]);
+        for (int r = 0; r < 2; r++) {
+#pragma unroll
+          for (int i = 0; i < (UPG == 1 ? 2 : 1); i++) s0[r][i] = scale_of(scr[0][r], i);
+#pragma unroll
+          for (int i = 0; i < (UPG == 1 ? NH2 : 1); i++) s1[r][i] = scale_of(scr[0][r], (UPG == 1 ? 2 : 1) + i);
+        }
+        uint8_t* Sx = Srow + 16 * x * ROWB;
+        unsigned short* SCx = SCrow + 16 * x * NG;
+        reg_fold_chunk<BITS, UPG, 2, NG, ROWB>(sw[0][0], sw[0][1], s0, A1, A2, A3, KBf, 0, lane, al2, Sx, SCx);
+        reg_fold_chunk<BITS, UPG, NH2, NG, ROWB>(sw[0][0] + 2 * WPU, sw[0][1] + 2 * WPU, s1, A1, A2, A3, KBf, 2, lane, al2, Sx, SCx);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+#pragma unroll
+          for (int p = 0; p < NU * WPU; p++) sw[0][r][p] = sw[1][r][p];
+#pragma unroll
+          for (int p = 0; p < (NG + 1) / 2; p++) scr[0][r][p] = scr[1][r][p];
+        }
       }
     }
   }
