@@ -350,8 +350,8 @@ __device__ __forceinline__ float fold_round(const float (&acc)[NH][4][4], int la
 // Bound by instruction issue (with its share of the step around it).  Two halves (64 columns, 32 values of a thread) are
 // taken at once: independent chains for the scheduler, and the 2 or 4 fresh scales of a quad (rows x groups) are
 // reduced by a transposing butterfly, computed by ONE lane each and exchanged.  Rounding is a branch-free exact division
-// (div_round2).  Token that folds, 256 rows of 32 heads, 8-bit: 123 us (141 us one span at a time with a verified reciprocal);
-// 4-bit, 4096 rows, a slot in eight folding: 767 us (941).
+// (div_round2).  One span at a time with a verified reciprocal the token that folds took a seventh longer (256 rows of 32 heads, 8-bit,
+// with the step kernel of then: 141 us, 123 so).
 template <int BITS, int UPG, int DV, bool VDEC = false, bool READ = false>
 __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short* scs, const int8_t* ubt, const float* udq,
                                                const float* tab, const float* ksf, const uint32_t* KBf, int w, int lane,
@@ -383,14 +383,10 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
       if constexpr (BITS == 8) {
 #pragma unroll
         for (int h = 0; h < NH; h++) ldsm_x4(m[h], addr ^ (32 * h));
-      } else if constexpr (NH == 2) {
+      } else {
         uint32_t x[4];
         ldsm_x4(x, addr);
         m[0][0] = x[0]; m[0][1] = x[1]; m[1][0] = x[2]; m[1][1] = x[3];
-      } else {
-        uint32_t x[2];
-        ldsm_x2(x, addr);
-        m[0][0] = x[0]; m[0][1] = x[1];
       }
       float sc[2][NS];
 #pragma unroll
@@ -421,16 +417,13 @@ __device__ __forceinline__ void fold_stage_mma(uint32_t st_addr, unsigned short*
       if constexpr (BITS == 8) {
 #pragma unroll
         for (int h = 0; h < NH; h++) stsm_x4(addr ^ (32 * h), o[h]);
-      } else if constexpr (NH == 2) {
+      } else {
         const uint32_t x[4] = {o[0][0], o[0][1], o[1][0], o[1][1]};
         stsm_x4(addr, x);
-      } else {
-        stsm_x2(addr, o[0][0], o[0][1]);
       }
     };
 #pragma unroll 1
     for (int h0 = 0; h0 + 2 <= NHALF; h0 += 2) chunk(IntC<2>(), h0);
-    if constexpr (NHALF % 2 == 1) chunk(IntC<1>(), NHALF - 1);
   };
 #pragma unroll 1
   for (int bb = 0; bb < 2; bb++) block(bb);

@@ -69,10 +69,11 @@ struct Residency {
 // Whether a step kernel of `grid` CTAs enters early, where the GPU holds `all`: the CTAs of two launches find room side by side up to
 // half of it, and from about 0.8 of it on they fill every SM however they come in.  Between the two they crowd on the SMs that are
 // free first.  us per layer-step in stream order / early, all slots due together: tensor-core kernel, int4 k/64 (740 at once) 320 CTAs
-// 7.0 / 6.7, 384 7.1 / 8.2, 576 8.1 / 8.5, 640 8.9 / 8.6, 1024 14.1 / 13.6; int8 v/32 (592) 288 CTAs 7.9 / 7.5, 304 8.5 / 9.1, 384 8.7 /
-// 9.2, 512 9.9 / 9.4; Mamba2 int8 320 7.3 / 6.8, 384 7.4 / 8.5, 640 9.9 / 9.5; register tile, int8 k/32 (592) 288 CTAs 4.3 / 4.0, 320 4.9 /
-// 5.5, 416 5.0 / 5.6, 512 5.9 / 5.6; bf16 1024 13.3 / 12.8.  KDA (one head per CTA: the folding ones end the launch) crowds up to a whole
-// wave where slots are due one in eight: 608 CTAs 12.1 / 12.9, 736 12.8 / 13.4 (all due 7.8 / 7.6, 8.3 / 7.8), 1024 17.6 / 17.4.
+// 6.4 / 6.0, 384 6.5 / 7.6, 576 7.6 / 7.9, 640 8.3 / 7.9, 1024 12.6 / 12.1; int8 v/32 (592) 288 CTAs 6.7 / 6.2, 304 7.4 / 8.3, 384 7.6 /
+// 8.3, 512 8.9 / 8.6; Mamba2 int8 320 6.5 / 6.0, 384 6.5 / 7.7, 640 8.6 / 8.3; register tile, int8 k/32 (592) 288 CTAs 4.3 / 3.9, 320 4.9 /
+// 5.2, 416 5.0 / 5.3, 512 5.7 / 5.3; bf16 1024 10.3 / 10.0.  KDA (one head per CTA: the folding ones end the launch) crowds up to a whole
+// wave where slots are due one in eight: int4 608 CTAs 11.3 / 12.2, 736 12.1 / 12.7 (all due 7.3 / 7.2, 7.9 / 7.4), 1024 (1036 at once)
+// 14.4 / 15.5.
 inline bool enters_early(long long grid, long long all, bool kda) { return 2 * grid <= all || (kda ? grid > all : 5 * grid > 4 * all); }
 
 // bf16 activations and output with q and k rows on 8-byte boundaries: the step kernels have instances of their own for these.

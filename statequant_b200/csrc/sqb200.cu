@@ -201,10 +201,10 @@ int launch(const sqb::StepArgs& a0, int bits, bool axk, cudaStream_t stream) {
   // (its CTAs are resident four to an SM).  There the serial chain of a CTA is what counts: it spreads a row over twice as many
   // warps (a head per CTA) and reads and folds without a detour through shared memory.  In longer grids its larger share of
   // per-CTA work counts.  us per layer and token, tensor-core kernel -> this one, slots folding together / an eighth of them on
-  // each token: int8 k/32, 32 heads of 128 x 128: 1 row 4.9 -> 3.3 / 5.0 -> 3.3, 8 rows 5.3 -> 4.1 / 12.3 -> 7.2, 18 rows (576 CTAs) 6.8
-  // -> 6.4 / 15.0 -> 9.8, 19 rows (608) 7.2 -> 8.6 / 14.2 -> 10.6, 37 rows 10.0 -> 11.5 / 21.9 -> 15.0; int4 k/64: 16 rows 6.3 -> 5.1 / 14.5 ->
-  // 8.2, 19 rows 6.7 -> 7.3 / 13.8 -> 9.3; Mamba2, 128 heads of 64 rows, int8: 8 rows (512) 7.1 -> 6.1 / 15.3 -> 9.1, 10 rows (640) 8.0 -> 8.7
-  // / 16.5 -> 10.6; int4: 6.2 -> 4.9 / 14.1 -> 8.1, 6.7 -> 7.6 / 15.0 -> 9.5.  In all four formats slots that fold together turn at one wave;
+  // each token: int8 k/32, 32 heads of 128 x 128: 1 row 4.6 -> 3.1 / 4.6 -> 3.1, 8 rows 4.9 -> 3.9 / 8.4 -> 5.8, 18 rows (576 CTAs) 5.6
+  // -> 5.4 / 9.9 -> 7.7, 19 rows (608) 6.0 -> 6.9 / 11.2 -> 8.8, 37 rows 8.0 -> 10.0 / 17.5 -> 13.2; int4 k/64: 16 rows 5.5 -> 5.0 / 9.7 ->
+  // 7.2, 19 rows 5.9 -> 6.8 / 11.1 -> 8.6; Mamba2, 128 heads of 64 rows, int8: 8 rows (512) 5.2 -> 5.1 / 9.6 -> 7.4, 10 rows (640) 5.9 -> 7.0
+  // / 9.5 -> 8.3; int4: 5.3 -> 4.7 / 9.7 -> 7.0, 5.9 -> 6.9 / 9.6 -> 8.1.  In all four formats slots that fold together turn at one wave;
   // where they do not is known to the device only.
   constexpr long long ONE_WAVE = 4 * SMS;
   if (path != 1 && sqb::reg_shape_ok(a0, bits, axk, KIND)) {
